@@ -340,6 +340,10 @@ int hydro3d_init_blast_at_f32(float *d_rhoE, float *d_uvw, size_t NB_X, size_t N
  * Synchronous. No counterpart in the reference. */
 int hydro_fused_math_f64(const double *d_x, size_t n, double *d_rcp, double *d_sqrt, void *stream);
 int hydro_fused_math_f32(const float *d_x, size_t n, float *d_rcp, float *d_sqrt, void *stream);
+/* The same as the strict arithmetic computes them for densities and squared impedances of
+ * ordinary size (2^-400 to 2^400 in FP64, 2^-60 to 2^60 in FP32): correctly rounded. */
+int hydro_strict_math_f64(const double *d_x, size_t n, double *d_rcp, double *d_sqrt, void *stream);
+int hydro_strict_math_f32(const float *d_x, size_t n, float *d_rcp, float *d_sqrt, void *stream);
 
 /* ---- errors -------------------------------------------------------------------------- */
 /* No counterpart in the reference (it has no status return): last error code latched

@@ -78,7 +78,16 @@ template <class T> __global__ void fused_math_kernel(const T *x, long long n, T 
     }
 }
 
-template <class T> int fused_math(const T *x, size_t n, T *rcp, T *sq, void *stream)
+// The same for the strict conversion's straight-line forms (regular inputs).
+template <class T> __global__ void strict_math_kernel(const T *x, long long n, T *rcp, T *sq)
+{
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        rcp[i] = Ex<T>::rcp(x[i]);
+        sq[i] = Ex<T>::sqrt(x[i]);
+    }
+}
+
+template <class T> int diag_math(void (*kern)(const T *, long long, T *, T *), const T *x, size_t n, T *rcp, T *sq, void *stream)
 {
     if (!x || !rcp || !sq) {
         set_error(kErrArg, "hydro_fused_math: null argument");
@@ -87,7 +96,7 @@ template <class T> int fused_math(const T *x, size_t n, T *rcp, T *sq, void *str
     if (n == 0) return kOk;
     const cudaStream_t st = (cudaStream_t)stream;
     const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)device_sms() * 8);
-    fused_math_kernel<T><<<blocks, 256, 0, st>>>(x, (long long)n, rcp, sq);
+    kern<<<blocks, 256, 0, st>>>(x, (long long)n, rcp, sq);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
@@ -103,11 +112,20 @@ extern "C" {
 
 int hydro_fused_math_f64(const double *d_x, size_t n, double *d_rcp, double *d_sqrt, void *stream)
 {
-    return fused_math<double>(d_x, n, d_rcp, d_sqrt, stream);
+    return diag_math<double>(fused_math_kernel<double>, d_x, n, d_rcp, d_sqrt, stream);
 }
 int hydro_fused_math_f32(const float *d_x, size_t n, float *d_rcp, float *d_sqrt, void *stream)
 {
-    return fused_math<float>(d_x, n, d_rcp, d_sqrt, stream);
+    return diag_math<float>(fused_math_kernel<float>, d_x, n, d_rcp, d_sqrt, stream);
+}
+
+int hydro_strict_math_f64(const double *d_x, size_t n, double *d_rcp, double *d_sqrt, void *stream)
+{
+    return diag_math<double>(strict_math_kernel<double>, d_x, n, d_rcp, d_sqrt, stream);
+}
+int hydro_strict_math_f32(const float *d_x, size_t n, float *d_rcp, float *d_sqrt, void *stream)
+{
+    return diag_math<float>(strict_math_kernel<float>, d_x, n, d_rcp, d_sqrt, stream);
 }
 
 double hydro2d_launcher_f64(const double *d_rhoE, const double *d_uv, double *d_rhoE_next, double *d_uv_next,

@@ -112,8 +112,10 @@ struct BatchAcc {
 struct MaxAcc {
     double vmax = 0.0;
     unsigned err = 0;
-    __device__ __forceinline__ void add_speed(double sp)
+    // a cell that the skip test does not pass (it passes positive densities only)
+    template <class T> __device__ __forceinline__ void add_speed(T rho, double sp)
     {
+        if (!(rho > T(0))) err |= kErrNonPhysical;
         vmax = (sp > vmax) ? sp : vmax;
         if (!(sp <= 1.0e300)) err |= kErrNonPhysical;
     }
@@ -402,9 +404,8 @@ __global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<
         const float tlo2 = skip_tlo2(batch_threshold(I, skip_frac)), ggm1 = I->ggm1;
         const bool ok = march2d<T, true, kF>(S, &I->tm[par][0], &I->tm[par][1], geo, I->rhoE[par ^ 1], I->uv[par ^ 1], ph,
                                    I->DtDx, I->DtDy, ld, [&](const Upd2<T> &o) {
-                                       if (!(o.r > T(0))) acc.err |= kErrNonPhysical;
                                        if (!state_below(o, ggm1, tlo2))
-                                           acc.add_speed((double)speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
+                                           acc.add_speed(o.r, (double)speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
                                    });
         if (!ok) acc.err |= kErrWaitTimeout;
         const int2 rg = ranges[it.x];
@@ -443,9 +444,8 @@ __global__ void __launch_bounds__(k3NT<T>, k3MinBlocks<T>) batch3d(Inst3<T> *ins
         march3d<T, kF, false, k3Warps<T>, false>(
             S, I->rhoE[par], I->uvw[par], I->rhoE[par ^ 1], I->uvw[par ^ 1], geo, ph, I->DtDx, I->DtDy, I->DtDz,
             [&](const Upd3<T> &o) {
-                if (!(o.r > T(0))) acc.err |= kErrNonPhysical;
                 if (!state_below(o, ggm1, tlo2))
-                    acc.add_speed((double)speed3<T, kF>(o.r, o.u, o.v, o.w, o.E, ph));
+                    acc.add_speed(o.r, (double)speed3<T, kF>(o.r, o.u, o.v, o.w, o.E, ph));
             });
         const int2 rg = ranges[it.x];
         if (publish_step<k3NT<T>>(acc, parts, w, &I->done_items, rg.y, &s_last))

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kStripNT, kMinB)
                                          [&](const Upd2<T> &o) {
                                              acc.add_mass(o.r);
                                              if (!state_below(o, ggm1, tlo2))
-                                                 acc.add_speed(speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
+                                                 acc.add_speed(o.r, speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
                                          });
     if (!ok) acc.err |= kErrWaitTimeout;
     step_epilogue<kStripNT, T>(acc, g.scr, g.partials, gridDim.x * gridDim.y, blockIdx.x + blockIdx.y * gridDim.x,

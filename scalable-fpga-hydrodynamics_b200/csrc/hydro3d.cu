@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(32 * W, min_blocks3<T>(W))
     auto sink = [&](const Upd3<T> &o) {
         acc.add_mass(o.r);
         if (!state_below(o, ggm1, tlo2))
-            acc.add_speed(speed3<T, kF>(o.r, o.u, o.v, o.w, o.E, ph));
+            acc.add_speed(o.r, speed3<T, kF>(o.r, o.u, o.v, o.w, o.E, ph));
     };
     bool ok;
     if constexpr (kPair)

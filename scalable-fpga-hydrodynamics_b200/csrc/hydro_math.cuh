@@ -38,6 +38,8 @@ template <> struct Ar<double> {
     static __device__ __forceinline__ double rcp(double a) { return __drcp_rn(a); }
     static __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
     static __device__ __forceinline__ double sqrt(double a) { return __dsqrt_rn(a); }
+    static __device__ __forceinline__ double abs(double a) { return fabs(a); }
+    static __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
     static constexpr double half = 0.5;
 };
 
@@ -48,6 +50,8 @@ template <> struct Ar<float> {
     static __device__ __forceinline__ float rcp(float a) { return __frcp_rn(a); }
     static __device__ __forceinline__ float div(float a, float b) { return __fdiv_rn(a, b); }
     static __device__ __forceinline__ float sqrt(float a) { return __fsqrt_rn(a); }
+    static __device__ __forceinline__ float abs(float a) { return fabsf(a); }
+    static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
     static constexpr float half = 0.5f;
 };
 
@@ -104,13 +108,17 @@ template <> struct Fu<float> {
         return m >= 0x1p-100f && m <= 0x1p100f;
     }
     static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-    static __device__ __forceinline__ float rcp(float a)
+    static __device__ __forceinline__ float rcp_reg(float a)
     {
-        if (!regular(a)) return __frcp_rn(a);
         float y;
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
         const float e = __fmaf_rn(-a, y, 1.0f);
         return __fmaf_rn(y, __fmaf_rn(e, e, e), y);
+    }
+    static __device__ __forceinline__ float rcp(float a)
+    {
+        if (!regular(a)) return __frcp_rn(a);
+        return rcp_reg(a);
     }
     static __device__ __forceinline__ float rsqrt_pos(float s)
     {
@@ -126,6 +134,73 @@ template <> struct Fu<float> {
     }
 };
 
+// Correctly rounded reciprocal and square root of regular inputs as straight-line code. The
+// intrinsics (__drcp_rn, __dsqrt_rn and the float forms) carry a branch to a special-case
+// path each, three per cell, which cut the block the scheduler can interleave; here the
+// cell conversion tests its two arguments once and recomputes the rare irregular cell with
+// the intrinsics (make_cell2 / make_cell3).
+//
+// Method: the refined approximation (Fu above), then one correction step with the exact
+// residual, which an fma gives without error (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990):
+//   1/a:     r = 1 - a y (exact),   y' = y + r y
+//   sqrt(s): r = s - g g (exact),   g' = g + r (y/2)
+// The correction's own error is below 2^-53 ulp (reciprocal) and 2^-50 ulp (square root), so
+// only an input whose exact result lies that close to a rounding midpoint could round the
+// wrong way: for the FP64 reciprocal the single significand 2 - 2^-52 (whose start value is
+// rounded away from the tie), for the FP64 square root the few dozen solutions of n 2^54 - q^2 = c and n 2^55 - q^2 = c with small c. The
+// tests enumerate these, and every FP32 significand.
+template <class T> struct Ex;
+
+template <> struct Ex<double> {
+    static __device__ __forceinline__ double rcp(double a)
+    {
+        double y0;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
+        const double e = __fma_rn(-a, y0, 1.0);
+        // rounded up: for the significand 2 - 2^-52 the correction from the lower neighbour
+        // would end in a tie
+        const double y = __fma_ru(y0, __fma_rn(e, e, e), y0);
+        return __fma_rn(__fma_rn(-a, y, 1.0), y, y);
+    }
+    static __device__ __forceinline__ double sqrt(double s)
+    {
+        const double y = Fu<double>::rsqrt_pos(s);
+        const double g = __dmul_rn(s, y);
+        return __fma_rn(__fma_rn(-g, g, s), __dmul_rn(0.5, y), g);
+    }
+    // exponent tests on the high word: density 2^-200 <= r < 2^200, squared impedance
+    // 2^-400 <= s < 2^400
+    static __device__ __forceinline__ bool regular(double r, double s)
+    {
+        return (unsigned)__double2hiint(r) - (823u << 20) < (400u << 20) &&
+               (unsigned)__double2hiint(s) - (623u << 20) < (800u << 20);
+    }
+};
+
+template <> struct Ex<float> {
+    static __device__ __forceinline__ float rcp(float a)
+    {
+        float y;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+        y = __fmaf_rn(__fmaf_rn(-a, y, 1.0f), y, y);
+        return __fmaf_rn(__fmaf_rn(-a, y, 1.0f), y, y);
+    }
+    static __device__ __forceinline__ float sqrt(float s)
+    {
+        float y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+        const float g = __fmul_rn(s, y), h = __fmul_rn(0.5f, y);
+        return __fmaf_rn(__fmaf_rn(-g, g, s), h, g);
+    }
+    // 2^-20 <= r < 2^20, 2^-40 <= s < 2^40
+    static __device__ __forceinline__ bool regular(float r, float s)
+    {
+        return (unsigned)__float_as_int(r) - (107u << 23) < (40u << 23) &&
+               (unsigned)__float_as_int(s) - (87u << 23) < (80u << 23);
+    }
+};
+
 template <class T> struct Vec2;
 template <> struct Vec2<double> { using type = double2; };
 template <> struct Vec2<float> { using type = float2; };
@@ -136,12 +211,14 @@ template <class T> __device__ __forceinline__ T smax(T a, T b) { return (a < b) 
 // Physical constants of one launch (hydro2d/kernel.hpp:63-68 argument list).
 template <class T> struct Phys {
     T C_min, gamma, gm1, divgamma, K;
-    bool kneg; // K < 0
-    T iK;      // 1 / K (fused arithmetic: 1/(K a) = (1/K)(1/a))
+    T iK;     // 1 / K (fused arithmetic: 1/(K a) = (1/K)(1/a))
+    bool odd; // K or gamma - 1 of no ordinary size: every cell takes the checked conversion
 
     static Phys make(T C_min, T gamma, T gm1, T divgamma, T K)
     {
-        return Phys{C_min, gamma, gm1, divgamma, K, K < T(0), T(1) / K};
+        const auto usual = [](T x) { return x > T(1.0 / 1048576) && x < T(1048576); };
+        return Phys{C_min, gamma, gm1, divgamma, K, T(1) / K,
+                    !(usual(K < T(0) ? -K : K) && usual(gamma) && usual(gm1) && usual(divgamma))};
     }
 };
 
@@ -180,43 +257,61 @@ template <class T> struct Cell2 {
     T r, u, v, p, Ka, iKa, mu, mv, eup;
 };
 
+// The conversion as one straight-line block for ordinary cells. `bad` says that density or
+// squared impedance gamma p rho lie outside the range where its values are those of
+// make_cell2_checked; make_cell2 recomputes such a cell with that, in one branch behind the
+// block. What bounds the marches is issue slots and latency: with the intrinsics' three
+// special-case branches per cell the strict march issued 329 instructions per 2D cell-update
+// at 8000 x 8000 FP64, so 294 (72.5 -> 79.3 GCell/s; FP32 107 -> 118). Recomputing behind the
+// x face instead keeps more values alive across it: 75.6 GCell/s.
+//
+// Strict: products by 1/2 are exact, so they move into an fma with the sum that follows
+// (E/rho - temp/2, and the 1/2 of the kinetic energy taken off the product r temp instead of
+// off r): the same rounding of the same value, one operation less each. A product so small
+// that 1/2 of it would round lies far below the ulp of the sum it enters.
 template <class T, bool kF = false>
-__device__ __forceinline__ Cell2<T> make_cell2_checked(T ur, T uu, T uv, T uE, const Phys<T> &ph);
-
-// FP64 fused arithmetic: one straight-line block (no branch inside the chain, so the
-// scheduler can interleave it with the face evaluations around it), then one warp-uniform
-// branch that recomputes the cells whose density or gamma p rho fell outside the range of
-// the refined approximations; the values equal make_cell2_checked's in every lane (2D
-// 88.2 -> 89.4 GCell/s fused at 40000 x 20000; the FP32 3D form measured slower and keeps
-// the checked path).
-template <class T, bool kF = false>
-__device__ __forceinline__ Cell2<T> make_cell2(T ur, T uu, T uv, T uE, const Phys<T> &ph)
+__device__ __forceinline__ Cell2<T> cell2_fast(T ur, T uu, T uv, T uE, const Phys<T> &ph, bool &bad)
 {
-    if constexpr (kF && sizeof(T) == 8) {
-        using A = Ar<T>;
-        using F = Fu<T>;
-        Cell2<T> c;
-        const T inv = F::rcp_reg(ur);
-        c.r = ur;
-        c.u = A::mul(uu, inv);
-        c.v = A::mul(uv, inv);
-        const T temp = F::fma(c.v, c.v, A::mul(c.u, c.u));
-        c.p = A::mul(A::mul(ph.gm1, ur), F::fma(-A::half, temp, A::mul(uE, inv)));
-        const T s = A::mul(A::mul(ph.gamma, c.p), c.r);
+    using A = Ar<T>;
+    using F = Fu<T>;
+    Cell2<T> c;
+    c.r = ur;
+    T inv;
+    if constexpr (kF) inv = F::rcp_reg(ur);
+    else inv = Ex<T>::rcp(ur);
+    c.u = A::mul(uu, inv);
+    c.v = A::mul(uv, inv);
+    T temp;
+    if constexpr (kF) temp = F::fma(c.v, c.v, A::mul(c.u, c.u));
+    else temp = A::add(A::mul(c.u, c.u), A::mul(c.v, c.v));
+    c.p = A::mul(A::mul(ph.gm1, ur), F::fma(-A::half, temp, A::mul(uE, inv)));
+    const T s = A::mul(A::mul(ph.gamma, c.p), c.r);
+    if constexpr (kF) {
         const T y = F::rsqrt_pos(s);
         c.Ka = A::mul(ph.K, A::mul(s, y));
         c.iKa = A::mul(ph.iK, y);
-        c.mu = A::mul(c.u, c.r);
-        c.mv = A::mul(c.v, c.r);
-        c.eup = F::fma(A::mul(A::half, c.r), temp, A::mul(c.p, ph.divgamma));
-        const bool bad = !F::regular(ur) || !(s > T(0) && F::regular(s));
-        if (__any_sync(__activemask(), bad)) {
-            if (bad) c = make_cell2_checked<T, true>(ur, uu, uv, uE, ph);
-        }
-        return c;
     } else {
-        return make_cell2_checked<T, kF>(ur, uu, uv, uE, ph);
+        c.Ka = A::mul(ph.K, Ex<T>::sqrt(s));
+        c.iKa = Ex<T>::rcp(c.Ka);
     }
+    c.mu = A::mul(c.u, c.r);
+    c.mv = A::mul(c.v, c.r);
+    if constexpr (kF) c.eup = F::fma(A::mul(A::half, c.r), temp, A::mul(c.p, ph.divgamma));
+    else c.eup = F::fma(A::half, A::mul(c.r, temp), A::mul(c.p, ph.divgamma));
+    bad = !Ex<T>::regular(ur, s) || ph.odd;
+    return c;
+}
+
+template <class T, bool kF = false>
+__device__ __forceinline__ Cell2<T> make_cell2_checked(T ur, T uu, T uv, T uE, const Phys<T> &ph);
+
+template <class T, bool kF = false>
+__device__ __forceinline__ Cell2<T> make_cell2(T ur, T uu, T uv, T uE, const Phys<T> &ph)
+{
+    bool bad;
+    Cell2<T> c = cell2_fast<T, kF>(ur, uu, uv, uE, ph, bad);
+    if (bad) c = make_cell2_checked<T, kF>(ur, uu, uv, uE, ph);
+    return c;
 }
 
 // The per-cell conversion with the range checks inside the chain (both arithmetics).
@@ -288,9 +383,9 @@ template <class T, bool kF = false>
 __device__ __forceinline__ Flux2<T> face_flux(const FaceIn<T> &L, const FaceIn<T> &R, const Phys<T> &ph)
 {
     using A = Ar<T>;
-    // std::max(a_left, a_right) takes a_right iff a_left < a_right; with K < 0 the
-    // products order the other way
-    const bool right = ph.kneg ? (R.Ka < L.Ka) : (L.Ka < R.Ka);
+    // std::max(a_left, a_right) takes a_right iff a_left < a_right; K < 0 flips the sign of
+    // both products, so their magnitudes order as a_left and a_right do for either sign
+    const bool right = A::abs(L.Ka) < A::abs(R.Ka);
     const T a = right ? R.Ka : L.Ka;
     const T diva = right ? R.iKa : L.iKa;
     if constexpr (kF) {
@@ -306,17 +401,20 @@ __device__ __forceinline__ Flux2<T> face_flux(const FaceIn<T> &L, const FaceIn<T
         return F2;
     }
     const T us = A::mul(A::half, A::sub(A::add(L.un, R.un), A::mul(diva, A::sub(R.p, L.p))));
-    const T ps = A::mul(A::half, A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un))));
+    // 2 p*: its 1/2 is exact and moves into the sums below
+    const T ps2 = A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un)));
     const bool up = us >= T(0);
     const T r = up ? L.r : R.r;
     const T mn = up ? L.mn : R.mn;
     const T mt = up ? L.mt : R.mt;
     const T e = up ? L.eup : R.eup;
     Flux2<T> F;
-    F.r = A::add(A::mul(r, us), T(0)); // "+ ZERO" kept: it turns -0 into +0
-    F.n = A::add(A::mul(mn, us), ps);
+    // the reference's "+ ZERO" turns -0 into +0: kept where a momentum of -0 would show it,
+    // left out where the flux enters the density (never -0 in a cell that has a finite 1/rho)
+    F.r = A::mul(r, us);
+    F.n = A::fma(A::half, ps2, A::mul(mn, us));
     F.t = A::add(A::mul(mt, us), T(0));
-    F.E = A::add(A::mul(e, us), A::mul(ps, us));
+    F.E = A::fma(A::half, A::mul(ps2, us), A::mul(e, us));
     return F;
 }
 
@@ -400,11 +498,18 @@ __device__ __forceinline__ bool speed_below(float r, float E, float m2, float gg
     if (!(r > 1e-6f) || !(r < 1e6f) || !(E > 1e-6f) || !(E < 1e12f) || !(m2 < 1e24f)) return false;
     return (ggm1 * E * r + m2) * (2.0f * (1.0f + 1.0f / 4096.0f)) < tlo2 * (r * r);
 }
-// The same test in FP64 for FP64 states (no conversions; the same bound, ranges and margin).
+// The same test in FP64 for FP64 states (no conversions). The ranges are tested on the high
+// words, in integer instructions beside the FP64 pipe's work: at most the ranges above (a
+// value between a bound and the next high word takes the exact path).
 __device__ __forceinline__ bool speed_below(double r, double E, double m2, double ggm1, double tlo2)
 {
-    if (!(r > 1e-6) || !(r < 1e6) || !(E > 1e-6) || !(E < 1e12) || !(m2 < 1e24)) return false;
-    return (ggm1 * E * r + m2) * (2.0 * (1.0 + 1.0 / 4096.0)) < tlo2 * (r * r);
+    constexpr unsigned lo = 0x3EB0C6F8u;  // the first high word above 1e-6
+    constexpr unsigned r_hi = 0x412E8480u; // 1e6
+    constexpr unsigned E_hi = 0x426D1A94u; // 1e12
+    constexpr unsigned m_hi = 0x44EA7843u; // 1e24
+    const bool in = (unsigned)__double2hiint(r) - lo < r_hi - lo && (unsigned)__double2hiint(E) - lo < E_hi - lo &&
+                    (unsigned)__double2hiint(m2) < m_hi;
+    return in && (ggm1 * E * r + m2) * (2.0 * (1.0 + 1.0 / 4096.0)) < tlo2 * (r * r);
 }
 // The skip test of a new 2D / 3D state in the state's own precision.
 template <class T> __device__ __forceinline__ bool state_below(const Upd2<T> &o, float ggm1, float tlo2)
@@ -436,43 +541,63 @@ template <class T> struct Cell3 {
     T r, u, v, w, p, Ka, iKa, mu, mv, mw, eup_xy, eup_z;
 };
 
+// As cell2_fast.
 template <class T, bool kF = false>
-__device__ __forceinline__ Cell3<T> make_cell3_checked(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph);
-
-// FP64 fused arithmetic: straight-line with a warp-uniform fix-up, as make_cell2 (3D 40.0 ->
-// 41.2 GCell/s fused at 512^3; FP32 62.7 against 63.4 with it, so FP32 keeps the checked
-// path).
-template <class T, bool kF = false>
-__device__ __forceinline__ Cell3<T> make_cell3(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph)
+__device__ __forceinline__ Cell3<T> cell3_fast(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph, bool &bad)
 {
-    if constexpr (kF && sizeof(T) == 8) {
-        using A = Ar<T>;
-        using F = Fu<T>;
-        Cell3<T> c;
-        const T inv = F::rcp_reg(ur);
-        c.r = ur;
-        c.u = A::mul(uu, inv);
-        c.v = A::mul(uv, inv);
-        c.w = A::mul(uw, inv);
-        const T temp = F::fma(c.w, c.w, F::fma(c.v, c.v, A::mul(c.u, c.u)));
-        c.p = A::mul(A::mul(ph.gm1, ur), F::fma(-A::half, temp, A::mul(uE, inv)));
-        const T s = A::mul(A::mul(ph.gamma, c.p), c.r);
+    using A = Ar<T>;
+    using F = Fu<T>;
+    Cell3<T> c;
+    c.r = ur;
+    T inv;
+    if constexpr (kF) inv = F::rcp_reg(ur);
+    else inv = Ex<T>::rcp(ur);
+    c.u = A::mul(uu, inv);
+    c.v = A::mul(uv, inv);
+    c.w = A::mul(uw, inv);
+    const T uu2 = A::mul(c.u, c.u);
+    T temp, tempz;
+    if constexpr (kF) {
+        temp = tempz = F::fma(c.w, c.w, F::fma(c.v, c.v, uu2));
+    } else {
+        const T vv2 = A::mul(c.v, c.v), ww2 = A::mul(c.w, c.w);
+        temp = A::add(A::add(uu2, vv2), ww2);
+        tempz = A::add(A::add(ww2, vv2), uu2);
+    }
+    c.p = A::mul(A::mul(ph.gm1, ur), F::fma(-A::half, temp, A::mul(uE, inv)));
+    const T s = A::mul(A::mul(ph.gamma, c.p), c.r);
+    if constexpr (kF) {
         const T y = F::rsqrt_pos(s);
         c.Ka = A::mul(ph.K, A::mul(s, y));
         c.iKa = A::mul(ph.iK, y);
-        c.mu = A::mul(c.u, c.r);
-        c.mv = A::mul(c.v, c.r);
-        c.mw = A::mul(c.w, c.r);
-        c.eup_xy = F::fma(A::mul(A::half, c.r), temp, A::mul(c.p, ph.divgamma));
-        c.eup_z = c.eup_xy;
-        const bool bad = !F::regular(ur) || !(s > T(0) && F::regular(s));
-        if (__any_sync(__activemask(), bad)) {
-            if (bad) c = make_cell3_checked<T, true>(ur, uu, uv, uw, uE, ph);
-        }
-        return c;
     } else {
-        return make_cell3_checked<T, kF>(ur, uu, uv, uw, uE, ph);
+        c.Ka = A::mul(ph.K, Ex<T>::sqrt(s));
+        c.iKa = Ex<T>::rcp(c.Ka);
     }
+    c.mu = A::mul(c.u, c.r);
+    c.mv = A::mul(c.v, c.r);
+    c.mw = A::mul(c.w, c.r);
+    const T eint = A::mul(c.p, ph.divgamma);
+    if constexpr (kF) {
+        c.eup_xy = c.eup_z = F::fma(A::mul(A::half, c.r), temp, eint);
+    } else {
+        c.eup_xy = F::fma(A::half, A::mul(c.r, temp), eint);
+        c.eup_z = F::fma(A::half, A::mul(c.r, tempz), eint);
+    }
+    bad = !Ex<T>::regular(ur, s) || ph.odd;
+    return c;
+}
+
+template <class T, bool kF = false>
+__device__ __forceinline__ Cell3<T> make_cell3_checked(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph);
+
+template <class T, bool kF = false>
+__device__ __forceinline__ Cell3<T> make_cell3(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph)
+{
+    bool bad;
+    Cell3<T> c = cell3_fast<T, kF>(ur, uu, uv, uw, uE, ph, bad);
+    if (bad) c = make_cell3_checked<T, kF>(ur, uu, uv, uw, uE, ph);
+    return c;
 }
 
 // The per-cell conversion with the range checks inside the chain (both arithmetics).
@@ -552,7 +677,7 @@ template <class T, bool kF = false>
 __device__ __forceinline__ Flux3<T> face_flux3(const FaceIn3<T> &L, const FaceIn3<T> &R, const Phys<T> &ph)
 {
     using A = Ar<T>;
-    const bool right = ph.kneg ? (R.Ka < L.Ka) : (L.Ka < R.Ka);
+    const bool right = A::abs(L.Ka) < A::abs(R.Ka);
     const T a = right ? R.Ka : L.Ka;
     const T diva = right ? R.iKa : L.iKa;
     if constexpr (kF) {
@@ -569,7 +694,7 @@ __device__ __forceinline__ Flux3<T> face_flux3(const FaceIn3<T> &L, const FaceIn
         return F3;
     }
     const T us = A::mul(A::half, A::sub(A::add(L.un, R.un), A::mul(diva, A::sub(R.p, L.p))));
-    const T ps = A::mul(A::half, A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un))));
+    const T ps2 = A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un))); // 2 p*, as in 2D
     const bool up = us >= T(0);
     const T r = up ? L.r : R.r;
     const T mn = up ? L.mn : R.mn;
@@ -577,11 +702,11 @@ __device__ __forceinline__ Flux3<T> face_flux3(const FaceIn3<T> &L, const FaceIn
     const T m2 = up ? L.mt2 : R.mt2;
     const T e = up ? L.eup : R.eup;
     Flux3<T> F;
-    F.r = A::add(A::mul(r, us), T(0));
-    F.n = A::add(A::mul(mn, us), ps);
+    F.r = A::mul(r, us);
+    F.n = A::fma(A::half, ps2, A::mul(mn, us));
     F.t1 = A::add(A::mul(m1, us), T(0));
     F.t2 = A::add(A::mul(m2, us), T(0));
-    F.E = A::add(A::mul(e, us), A::mul(ps, us));
+    F.E = A::fma(A::half, A::mul(ps2, us), A::mul(e, us));
     return F;
 }
 

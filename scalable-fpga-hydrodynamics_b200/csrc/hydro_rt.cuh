@@ -175,16 +175,22 @@ struct StepAcc {
     template <class T> __device__ __forceinline__ void add_cell(T rho_new, T speed)
     {
         add_mass(rho_new);
-        add_speed(speed);
+        add_speed(rho_new, speed);
     }
     template <class T> __device__ __forceinline__ void add_mass(T rho_new)
     {
-        if (!(rho_new > T(0))) err |= kErrNonPhysical;
         // Kahan step, branch-free; mc carries the low part to add back (mass = ms + mc)
         const double y = __dadd_rn(static_cast<double>(rho_new), mc);
         const double tt = __dadd_rn(ms, y);
         mc = __dsub_rn(y, __dsub_rn(tt, ms));
         ms = tt;
+    }
+    // the exact signal speed of a cell, and the checks of the cells that the skip test does
+    // not pass (it passes positive densities only)
+    template <class T> __device__ __forceinline__ void add_speed(T rho_new, T speed)
+    {
+        if (!(rho_new > T(0))) err |= kErrNonPhysical;
+        add_speed(speed);
     }
     template <class T> __device__ __forceinline__ void add_speed(T speed)
     {

@@ -150,8 +150,12 @@ template <class SM> __device__ __forceinline__ void march3d_init(SM &S)
 // straight-line block ahead of the plane's barrier: independent chains the scheduler
 // interleaves; after the barrier only the update of plane m-1 remains. (Converting first
 // and evaluating the faces after the stage wait of the next plane measured 33.3 against
-// 35.3 GCell/s strict at 512^3 with 8-row tiles; the 9-row tile 37.2.) Returns false when a
-// bounded barrier wait gave up.
+// 35.3 GCell/s strict at 512^3 with 8-row tiles.) The loop is not unrolled: two planes of it
+// and the halo warp's loop beside them are about 20 KB of instructions, more than the SM's
+// instruction cache keeps (stall_no_instruction 0.86 cycles per issue against 0.24), and the
+// moves of the plane's values into the previous plane's registers cost less: 36.8 -> 39.4
+// GCell/s strict at 512^3, 29.7 -> 33.9 at 256^3. Returns false when a bounded barrier wait
+// gave up.
 template <bool kEdge, bool kF, class SM, class T, class Sink>
 __device__ __forceinline__ bool march3d_tma(SM &S, T *rhoE_n, T *uvw_n, const March3 &g, const Phys<T> &ph, T DtDx,
                                             T DtDy, T DtDz, const Tmaps3 &tm, Sink &sink)
@@ -267,7 +271,7 @@ __device__ __forceinline__ bool march3d_tma(SM &S, T *rhoE_n, T *uvw_n, const Ma
             Ur = ur; Uu = uu; Uv = uv; Uw = uw; UE = uE;
         }
         if (!aborted) {
-#pragma unroll 2
+#pragma unroll 1
             for (; m < nplanes; ++m) {
                 T ur, uE, uu, uv, uw;
                 wait(m);
@@ -529,12 +533,12 @@ __device__ __forceinline__ bool march3d_lane(Smem3<T, W> &S, const T *rhoE, cons
     return true;
 }
 
-// Per-lane copies, strict FP64: the plane loop written once per warp role, with the
-// interior rows' +y / +z faces of plane m-1, conversion of plane m and x face in one block
-// ahead of the barrier, as in the tensor-map form (FP64 with an odd NB_Z, 512 x 512 x 511:
-// 31.3 -> 34.0 GCell/s, no spills against 12 bytes). FP32 keeps march3d_lane: this form
-// ran 56.0 -> 57.2 GCell/s strict at 512^3 but 0.407 -> 0.454 ms at 256^3 (short chunks);
-// in fused arithmetic it measured slower (FP32 63.6 -> 60.4, FP64 35.9 -> 30.7 with spills).
+// Per-lane copies, FP64: the plane loop written once per warp role, with the interior rows'
+// +y / +z faces of plane m-1, conversion of plane m and x face in one block ahead of the
+// barrier, and not unrolled, as in the tensor-map form (FP64 with an odd NB_Z, 512 x 512 x
+// 511: strict 34.0 GCell/s, 23.9 unrolled by two, where it spills; fused 36.7 against 35.4 with
+// march3d_lane). FP32 keeps march3d_lane: this form runs 67.6 -> 67.0 GCell/s fused at 512^3
+// and 53.4 -> 48.3 at 256^3.
 template <bool kEdge, bool kF, class T, int W, class Sink>
 __device__ __forceinline__ bool march3d_lane_roles(Smem3<T, W> &S, const T *rhoE, const T *uvw, T *rhoE_n, T *uvw_n,
                                                const March3 &g, const Phys<T> &ph, T DtDx, T DtDy, T DtDz, Sink &sink)
@@ -657,7 +661,7 @@ __device__ __forceinline__ bool march3d_lane_roles(Smem3<T, W> &S, const T *rhoE
             Pm = P;
             Ur = ur; Uu = uu; Uv = uv; Uw = uw; UE = uE;
         }
-#pragma unroll 2
+#pragma unroll 1
         for (; m < nplanes; ++m) {
             T ur, uE, uu, uv, uw;
             load(m, ur, uE, uu, uv, uw);
@@ -716,7 +720,7 @@ __device__ __forceinline__ bool march3d_lane_roles(Smem3<T, W> &S, const T *rhoE
 // One tile march: the lean form for tiles away from walls and ghosts, the general one
 // elsewhere (the choice is uniform over the block). kF: fused arithmetic (hydro_math.cuh).
 // kTma: planes staged by the tensor maps `tm` (march3d_init first); else per-lane copies
-// (march3d_lane_roles in strict FP64 when kLaneRoles, else march3d_lane; the batched
+// (march3d_lane_roles in FP64 when kLaneRoles, else march3d_lane; the batched
 // engine keeps march3d_lane, where the role split spills in its persistent loop).
 // Returns false when a bounded barrier wait gave up.
 template <class T, bool kF = false, bool kTma = false, int W = k3Warps<T>, bool kLaneRoles = true, class Sink>
@@ -729,7 +733,7 @@ __device__ __forceinline__ bool march3d(Smem3<T, W> &S, const T *rhoE, const T *
         if (inner) return march3d_tma<false, kF>(S, rhoE_n, uvw_n, g, ph, DtDx, DtDy, DtDz, tm, sink);
         return march3d_tma<true, kF>(S, rhoE_n, uvw_n, g, ph, DtDx, DtDy, DtDz, tm, sink);
     } else {
-        if constexpr (!kF && kLaneRoles && sizeof(T) == 8) {
+        if constexpr (kLaneRoles && sizeof(T) == 8) {
             if (inner) return march3d_lane_roles<false, kF>(S, rhoE, uvw, rhoE_n, uvw_n, g, ph, DtDx, DtDy, DtDz, sink);
             return march3d_lane_roles<true, kF>(S, rhoE, uvw, rhoE_n, uvw_n, g, ph, DtDx, DtDy, DtDz, sink);
         } else {
