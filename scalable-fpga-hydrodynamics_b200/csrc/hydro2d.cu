@@ -286,18 +286,12 @@ template <> CUtensorMapDataType tmap_type<float>() { return CU_TENSOR_MAP_DATA_T
 bool aligned(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 } // namespace
 
-template <class T, int kMinB>
-void launch_strip2d(bool tma, bool fused, dim3 grid, cudaStream_t stream, const CUtensorMap &tmr,
-                    const CUtensorMap &tmu, const Args2<T> &g)
+template <class T> using Strip2 = void (*)(const CUtensorMap, const CUtensorMap, Args2<T>);
+
+template <class T, int kMinB> Strip2<T> strip2d_form(bool tma, bool fused)
 {
-    if (tma && fused)
-        strip2d<T, true, true, kMinB><<<grid, kStripNT, 0, stream>>>(tmr, tmu, g);
-    else if (tma)
-        strip2d<T, true, false, kMinB><<<grid, kStripNT, 0, stream>>>(tmr, tmu, g);
-    else if (fused)
-        strip2d<T, false, true, kMinB><<<grid, kStripNT, 0, stream>>>(tmr, tmu, g);
-    else
-        strip2d<T, false, false, kMinB><<<grid, kStripNT, 0, stream>>>(tmr, tmu, g);
+    if (tma) return fused ? strip2d<T, true, true, kMinB> : strip2d<T, true, false, kMinB>;
+    return fused ? strip2d<T, false, true, kMinB> : strip2d<T, false, false, kMinB>;
 }
 
 template <class T>
@@ -367,16 +361,20 @@ int step2d(const T *rhoE, const T *uv, T *rhoE_next, T *uv_next, T *Dt_next, con
     unsigned nblocks;
     if (use_strip) {
         const int nstrips = (int)((nb_y + kStripW - 1) / kStripW);
-        // rows per block: sized for about 24 blocks per SM, at least 16 and at most the cap
-        // (the tuned value when one is set with hydro_set_launch_shape, else 256), so that
-        // small grids still fill the GPU
+        // rows per block: at most the cap (the tuned value when one is set with
+        // hydro_set_launch_shape, else 256), at least 2 (one row per block measured no faster)
         const LaunchShape shape = launch_shape(2, sizeof(T));
-        const int cap = shape.chunk > 0 ? shape.chunk : 256;
-        const int target = device_sms() * 3 * 8;
-        int nchunks = (target + nstrips - 1) / nstrips;
-        int chunk = (int)((nb_x + nchunks - 1) / nchunks);
-        chunk = std::min(cap, std::max(std::min(16, cap), chunk));
-        nchunks = (int)((nb_x + chunk - 1) / chunk);
+        constexpr int kAltB = sizeof(T) == 8 ? 5 : 8; // the other register budget built
+        const bool alt = shape.blocks == kAltB;
+        const Strip2<T> kern = alt ? strip2d_form<T, kAltB>(tma_ok, fused) : strip2d_form<T, 4>(tma_ok, fused);
+        int per_sm = 1;
+        cudaError_t eo = blocks_per_sm(reinterpret_cast<const void *>(kern), kStripNT, 0, &per_sm);
+        if (eo != cudaSuccess) {
+            set_error(kErrCuda, "step2d: %s", cudaGetErrorString(eo));
+            return kErrCuda;
+        }
+        int chunk = march_chunk(nb_x, (size_t)nstrips, per_sm, shape.chunk > 0 ? shape.chunk : 256, 2);
+        int nchunks = (int)((nb_x + chunk - 1) / chunk);
         if (nchunks > 65535) {
             chunk = (int)((nb_x + 65534) / 65535);
             nchunks = (int)((nb_x + chunk - 1) / chunk);
@@ -389,13 +387,8 @@ int step2d(const T *rhoE, const T *uv, T *rhoE_next, T *uv_next, T *Dt_next, con
         ctx->last_chunk = chunk;
         ctx->last_tma = tma_ok;
         const dim3 grid(nstrips, nchunks);
-        constexpr int kAltB = sizeof(T) == 8 ? 5 : 8; // the other register budget built
-        const bool alt = shape.blocks == kAltB;
         ctx->last_blocks = alt ? kAltB : 4;
-        if (alt)
-            launch_strip2d<T, kAltB>(tma_ok, fused, grid, stream, tmr, tmu, g);
-        else
-            launch_strip2d<T, 4>(tma_ok, fused, grid, stream, tmr, tmu, g);
+        kern<<<grid, kStripNT, 0, stream>>>(tmr, tmu, g);
     } else {
         const int gx = (int)((nb_y + kDirectNT - 1) / kDirectNT);
         const int gy = (int)std::min<size_t>(nb_x, 65535);

@@ -164,27 +164,39 @@ template <class T> constexpr bool tile3_built(int rows)
 // 35.3 GCell/s strict at 512^3 for 8 rows), else 8.
 template <class T> int default_rows3(bool tma) { return (sizeof(T) == 8 && tma) ? 9 : k3Warps<T>; }
 
-template <class T, int W, bool kPair = false>
-cudaError_t launch_strip3d(bool fused, bool tma, dim3 grid, cudaStream_t stream, const CUtensorMap &tmr,
-                           const CUtensorMap &tmu, const Args3<T> &g)
+// A built form of the step: the kernel, its threads and its dynamic shared memory.
+template <class T> struct Form3 {
+    void (*kern)(const CUtensorMap, const CUtensorMap, Args3<T>) = nullptr;
+    int threads = 0, smem = 0;
+};
+
+template <class T, int W, bool kPair = false> Form3<T> strip3d_form(bool fused, bool tma)
 {
-    void (*kern)(const CUtensorMap, const CUtensorMap, Args3<T>);
-    int smem;
+    Form3<T> f;
+    f.threads = 32 * W;
     if constexpr (kPair) {
-        kern = fused ? strip3d<T, true, true, W, true> : strip3d<T, false, true, W, true>;
-        smem = (int)sizeof(Smem3P<T>);
+        f.kern = fused ? strip3d<T, true, true, W, true> : strip3d<T, false, true, W, true>;
+        f.smem = (int)sizeof(Smem3P<T>);
     } else {
         if constexpr (sizeof(T) == 8)
-            kern = fused ? (tma ? strip3d<T, true, true, W> : strip3d<T, true, false, W>)
-                         : (tma ? strip3d<T, false, true, W> : strip3d<T, false, false, W>);
+            f.kern = fused ? (tma ? strip3d<T, true, true, W> : strip3d<T, true, false, W>)
+                           : (tma ? strip3d<T, false, true, W> : strip3d<T, false, false, W>);
         else
-            kern = fused ? strip3d<T, true, false, W> : strip3d<T, false, false, W>;
-        smem = (int)sizeof(Smem3<T, W>);
+            f.kern = fused ? strip3d<T, true, false, W> : strip3d<T, false, false, W>;
+        f.smem = (int)sizeof(Smem3<T, W>);
     }
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, 32 * W, smem, stream>>>(tmr, tmu, g);
-    return cudaGetLastError();
+    return f;
+}
+
+// The form of a tile height: 9 rows run on 8 warps (FP64 tensor maps only), others on one
+// warp per row.
+template <class T> Form3<T> form3(int rows, bool fused, bool tma)
+{
+    if constexpr (sizeof(T) == 8) {
+        if (rows == 9) return strip3d_form<T, 8, true>(fused, true);
+        if (rows == 12) return strip3d_form<T, 12>(fused, tma);
+    }
+    return rows == 8 ? strip3d_form<T, 8>(fused, tma) : strip3d_form<T, 16>(fused, tma);
 }
 
 // ------------------------------------------------------------- initial condition ---
@@ -320,14 +332,16 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
             set_error(kErrArg, "step3d: NB_Y %zu too large for the strip kernel", nb_y);
             return kErrArg;
         }
-        // planes per block: sized for about 8 waves of resident blocks, at least 8 and at
-        // most the cap (the tuned value when one is set, else 256)
-        const int cap = shape.chunk > 0 ? shape.chunk : 256;
-        const int target = device_sms() * min_blocks3<T>(W) * 8;
-        int nchunks = std::max(1, (target + nz * ny - 1) / (nz * ny));
-        int chunk = (int)((nb_x + nchunks - 1) / nchunks);
-        chunk = std::min(cap, std::max(std::min(8, cap), chunk));
-        nchunks = (int)((nb_x + chunk - 1) / chunk);
+        // planes per block: at most the cap (the tuned value when one is set, else 256)
+        const Form3<T> form = form3<T>(rows, fused, tma);
+        int per_sm = 1;
+        cudaError_t ea = blocks_per_sm(reinterpret_cast<const void *>(form.kern), form.threads, form.smem, &per_sm);
+        if (ea != cudaSuccess) {
+            set_error(kErrCuda, "step3d: %s", cudaGetErrorString(ea));
+            return kErrCuda;
+        }
+        int chunk = march_chunk(nb_x, (size_t)nz * ny, per_sm, shape.chunk > 0 ? shape.chunk : 256, 3);
+        int nchunks = (int)((nb_x + chunk - 1) / chunk);
         if (nchunks > 65535) {
             chunk = (int)((nb_x + 65534) / 65535);
             nchunks = (int)((nb_x + chunk - 1) / chunk);
@@ -345,28 +359,14 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
                                  64, (uint32_t)rows, 1) &&
                   encode_tmap_3d(&tmu, tmap_type3<T>(), uvw, 3 * zs, ys, xs, 3 * zs * sizeof(T), 3 * zs * ys * sizeof(T),
                                  96, (uint32_t)rows, 1);
-            if (!tma && rows == 9) {
-                set_error(kErrCuda, "step3d: tensor maps of the 9-row tile rejected");
+            if (!tma) {
+                set_error(kErrCuda, "step3d: tensor maps rejected");
                 return kErrCuda;
             }
         }
         const dim3 grid(nz, ny, nchunks);
-        cudaError_t ea;
-        if (rows == 9) {
-            if constexpr (sizeof(T) == 8)
-                ea = launch_strip3d<T, 8, true>(fused, true, grid, stream, tmr, tmu, g);
-            else
-                ea = cudaErrorInvalidValue;
-        } else if (W == 8) {
-            ea = launch_strip3d<T, 8>(fused, tma, grid, stream, tmr, tmu, g);
-        } else if constexpr (sizeof(T) == 8) {
-            if (W == 12)
-                ea = launch_strip3d<T, 12>(fused, tma, grid, stream, tmr, tmu, g);
-            else
-                ea = launch_strip3d<T, 16>(fused, tma, grid, stream, tmr, tmu, g);
-        } else {
-            ea = launch_strip3d<T, 16>(fused, tma, grid, stream, tmr, tmu, g);
-        }
+        form.kern<<<grid, form.threads, form.smem, stream>>>(tmr, tmu, g);
+        ea = cudaGetLastError();
         if (ea != cudaSuccess) {
             ctx->dirty = true;
             set_error(kErrCuda, "step3d launch: %s", cudaGetErrorString(ea));

@@ -89,6 +89,13 @@ int ctx_count();
 // Streaming multiprocessors of the current device, queried once per device (launch
 // shapes are sized in multiples of it); 1 if the query fails.
 int device_sms();
+// Resident blocks per SM of a kernel on the current device, asked for once per kernel and
+// device; the first call also allows the kernel its `smem` bytes of dynamic shared memory.
+cudaError_t blocks_per_sm(const void *kernel, int threads, int smem, int *blocks);
+// Rows (2D) or planes (3D) that each block of a march takes: `rows` of them over `tiles`
+// columns of blocks, `per_sm` resident blocks per SM, at most `cap` and at least `least` rows
+// per block (context.cu).
+int march_chunk(size_t rows, size_t tiles, int per_sm, int cap, int least);
 // Grow the partials array to at least n entries (synchronises the device on growth).
 int ctx_reserve(DevCtx *c, size_t n);
 
