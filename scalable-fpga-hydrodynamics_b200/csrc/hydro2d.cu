@@ -55,14 +55,6 @@ template <class T> struct Args2 {
     int xwrap;              // X neighbours by periodic wrap (1) or from the ghost rows (0)
 };
 
-// The float skip threshold, rounded down so that every skipped cell is provably below
-// the double threshold the last block checks against.
-__device__ __forceinline__ float skip_threshold_f(const StepScratch *scr, unsigned long long key)
-{
-    return __double2float_rd(skip_threshold(scr, key));
-}
-
-
 // ------------------------------------------------------------------ direct kernel ---
 constexpr int kDirectNT = 128;
 
@@ -134,8 +126,8 @@ __global__ void __launch_bounds__(kStripNT, kMinB)
     const March2 geo{kStripW * (int)blockIdx.x, i0, min(i0 + g.chunk - 1, g.nb_x), g.nb_x, g.nb_y, g.ys, g.xwrap,
                      g.rhoE, g.uv};
     StepAcc acc;
-    const float tlof = skip_threshold_f(g.scr, g.key);
-    const float tlo2 = skip_tlo2(tlof), ggm1 = g.ggm1;
+    const SkipLimits lim = skip_limits(g.scr, g.key);
+    const float tlo2 = skip_tlo2(lim.f), ggm1 = g.ggm1;
     const Phys<T> ph = g.ph;
     unsigned ld = 0;
     const bool ok = march2d<T, kTma, kF>(S, &tmr, &tmu, geo, g.rhoE_n, g.uv_n, ph, g.DtDx, g.DtDy, ld,
@@ -146,7 +138,7 @@ __global__ void __launch_bounds__(kStripNT, kMinB)
                                          });
     if (!ok) acc.err |= kErrWaitTimeout;
     step_epilogue<kStripNT, T>(acc, g.scr, g.partials, gridDim.x * gridDim.y, blockIdx.x + blockIdx.y * gridDim.x,
-                               g.ph.C_min, g.Dt_next, g.status, g.seq, (double)tlof, g.key);
+                               g.ph.C_min, g.Dt_next, g.status, g.seq, (double)lim.hist, g.key);
 }
 
 // ------------------------------------------------------------- initial condition ---

@@ -133,8 +133,8 @@ __global__ void __launch_bounds__(32 * W, min_blocks3<T>(W))
     const March3 geo{k3TZ * (int)blockIdx.x, (kRows - 2) * (int)blockIdx.y, i0, min(i0 + g.chunk - 1, g.nb_x),
                      g.nb_x, g.nb_y, g.nb_z, g.zs, g.zy, g.xwrap};
     StepAcc acc;
-    const float tlof = __double2float_rd(skip_threshold(g.scr, g.key));
-    const float tlo2 = skip_tlo2(tlof), ggm1 = g.ggm1;
+    const SkipLimits lim = skip_limits(g.scr, g.key);
+    const float tlo2 = skip_tlo2(lim.f), ggm1 = g.ggm1;
     const Phys<T> ph = g.ph;
     auto sink = [&](const Upd3<T> &o) {
         acc.add_mass(o.r);
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(32 * W, min_blocks3<T>(W))
     if (!ok) acc.err |= kErrWaitTimeout;
     step_epilogue<32 * W, T>(acc, g.scr, g.partials, gridDim.x * gridDim.y * gridDim.z,
                              blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), g.ph.C_min, g.Dt_next,
-                             g.status, g.seq, (double)tlof, g.key);
+                             g.status, g.seq, (double)lim.hist, g.key);
 }
 
 // Tile heights (rows with halo) the plain 3D step is built for: FP64 8, 9 (8 warps, warp 0

@@ -63,6 +63,20 @@ __device__ __forceinline__ double skip_threshold(const StepScratch *scr, unsigne
     return (key != 0ull && k == key) ? kSkipFrac * m : 0.0;
 }
 
+// The thresholds of one block: `hist` from the previous step, checked against this step's max
+// at its end, and `f` for the skip test, raised to the max that the launch's finished blocks
+// have reached so far: a cell below that cannot hold the max, whatever the history says. Both
+// rounded down to float, so that every skipped cell is provably below the value in double.
+struct SkipLimits {
+    float hist, f;
+};
+__device__ __forceinline__ SkipLimits skip_limits(const StepScratch *scr, unsigned long long key)
+{
+    const unsigned long long m = *reinterpret_cast<const volatile unsigned long long *>(&scr->max_bits);
+    const double h = skip_threshold(scr, key), now = __longlong_as_double((long long)m);
+    return SkipLimits{__double2float_rd(h), __double2float_rd(h > now ? h : now)};
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
