@@ -198,9 +198,8 @@ unsigned hydro2d_noalloc_launch_shape(size_t NB_X, size_t NB_Y, int strip, int s
  * autotuner picks it. 0 keeps the built-in choice for any field.
  *  warps: 3D only, the tile height in rows with the one-row halo (8, 16, and in FP64 also
  *    9 and 12). Tiles of 8, 12 and 16 rows run one warp per row; a 9-row tile runs on 8
- *    warps, warp 0 holding both halo rows, and needs the tensor-map staging (FP64 with an
- *    even NB_Z and 16-byte aligned arrays; elsewhere 8 rows run). Built-in: 9 where the
- *    tensor maps apply, else 8;
+ *    warps, warp 0 holding both halo rows. Built-in: 9, which also runs for arrays that are not
+ *    all 16-byte aligned;
  *  chunk: the most rows (2D) or planes (3D) one block marches (built-in 256); blocks take
  *    fewer on grids too small to fill the GPU with that many (sized from the grid and the
  *    SM count);
@@ -284,7 +283,7 @@ typedef struct hydro_batch_status {
 } hydro_batch_status_t;
 
 /* A batch of `dim`-D (2) instances in FP32 (precision_bytes 4) or FP64 (8), rows per work
- * item `chunk` (0: 32 rows in 2D, 64 planes in 3D), at most `capacity` instances, on `stream`
+ * item `chunk` (0: chosen for the instances at hand), at most `capacity` instances, on `stream`
  * (NULL: its own). */
 void *hydro_batch_create(int dim, int precision_bytes, int chunk, int capacity, void *stream);
 /* Allocate, initialise and admit one instance; returns its slot (>= 0) or an error code. */

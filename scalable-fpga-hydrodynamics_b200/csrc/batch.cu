@@ -7,7 +7,7 @@
 // (strip2d_march.cuh / strip3d_march.cuh), so an instance's state after n batched steps
 // is bit-identical to n plain steps in the same precision. 2D instances keep the pair
 // layout with rows padded to 16 bytes (TMA-fed); 3D instances keep the reference's
-// pair/triple layout (cp.async-fed). Work is a flat list of (instance, tile x chunk)
+// pair/triple layout (row copies). Work is a flat list of (instance, tile x chunk)
 // items; persistent blocks take items from an atomic counter. Every item writes its max
 // signal speed and error bits to its own slot; the item that completes an instance's
 // step (ticket per instance) merges that instance's slots -- the result depends neither
@@ -48,7 +48,7 @@ template <class T> struct alignas(128) Inst2 {
     unsigned sum_items; // items of the end-of-run conservation sums done
     long long ys;
     long long steps, max_steps;
-    int nb_x, nb_y, nstrips, chunk;
+    int nb_x, nb_y, nstrips;
     int parity, active;
     unsigned done_items, err;
 };
@@ -64,9 +64,15 @@ template <class T> struct alignas(128) Inst3 {
     unsigned sum_items; // items of the end-of-run conservation sums done
     long long zs, zy;
     long long steps, max_steps;
-    int nb_x, nb_y, nb_z, ntz, nty, chunk;
+    int nb_x, nb_y, nb_z, ntz, nty;
     int parity, active;
     unsigned done_items, err;
+};
+
+// An instance's share of the work lists: its step items (parts slots first .. first+count-1, each
+// `chunk` rows or planes of a strip or tile) and its items of the end-of-run sums.
+struct Range {
+    int first, count, chunk, sum_first, sum_count;
 };
 
 struct ItemPart {
@@ -373,7 +379,7 @@ template <class T> struct Batch2dOcc { static constexpr int value = sizeof(T) ==
 
 // kF: fused arithmetic (hydro_math.cuh)
 template <class T, bool kF>
-__global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<T> *insts, const int2 *items, const int2 *ranges,
+__global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<T> *insts, const int2 *items, const Range *ranges,
                                                       int nitems, unsigned *counter, ItemPart *parts,
                                                       SlotStatus *status, double skip_frac)
 {
@@ -391,10 +397,11 @@ __global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<
         const int2 it = items[w];
         Inst2<T> *I = insts + it.x;
         if (!I->active) continue;
+        const Range rg = ranges[it.x];
         const int par = I->parity;
         const int strip = it.y % I->nstrips, ck = it.y / I->nstrips;
-        const int i0 = 1 + ck * I->chunk;
-        const March2 geo{kStripW * strip, i0, min(i0 + I->chunk - 1, I->nb_x), I->nb_x, I->nb_y, I->ys, 1};
+        const int i0 = 1 + ck * rg.chunk;
+        const March2 geo{kStripW * strip, i0, min(i0 + rg.chunk - 1, I->nb_x), I->nb_x, I->nb_y, I->ys, 1};
         const Phys<T> ph = I->ph;
         if (threadIdx.x == 0) {
             prefetch_tensormap(&I->tm[par][0]);
@@ -408,85 +415,160 @@ __global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<
                                            acc.add_speed(o.r, (double)speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
                                    });
         if (!ok) acc.err |= kErrWaitTimeout;
-        const int2 rg = ranges[it.x];
-        if (publish_step<kStripNT>(acc, parts, w, &I->done_items, rg.y, &s_last))
-            finalize_step<kStripNT, T, kF>(I, parts + rg.x, rg.y, status ? status + it.x : nullptr, skip_frac);
+        if (publish_step<kStripNT>(acc, parts, w, &I->done_items, rg.count, &s_last))
+            finalize_step<kStripNT, T, kF>(I, parts + rg.first, rg.count, status ? status + it.x : nullptr, skip_frac);
     }
 }
+
+// The tile of the 3D batch: 9 rows on 8 warps, planes by row copies (any NB_Z).
+template <class T> using Tile3 = Smem3<T, 8, true, Stage3::Rows>;
+template <class T> constexpr int k3NT = 32 * Tile3<T>::W;
+template <class T> constexpr int k3TY = Tile3<T>::R - 2; // interior rows per tile
 
 template <class T, bool kF>
-__global__ void __launch_bounds__(k3NT<T>, k3MinBlocks<T>) batch3d(Inst3<T> *insts, const int2 *items, const int2 *ranges,
-                                                  int nitems, unsigned *counter, ItemPart *parts,
-                                                  SlotStatus *status, double skip_frac)
+__global__ void __launch_bounds__(k3NT<T>, min_blocks3<T>(8)) batch3d(Inst3<T> *insts, const int2 *items,
+                                                                      const Range *ranges, int nitems, unsigned *counter,
+                                                                      ItemPart *parts, SlotStatus *status, double skip_frac)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem3<T> &S = *reinterpret_cast<Smem3<T> *>(smem_raw);
-    __shared__ int s_item;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    Tile3<T> &S = *reinterpret_cast<Tile3<T> *>(smem_raw);
+    // the item at hand, its instance's grid and constants: read again where they are needed. Held
+    // in registers through the march they cost about 30 of its 128, and it spilled: 8 steps of
+    // 15.8 M cells FP64 took 6.6 ms, so 4.7 ms (5.2 ms with the former march).
+    struct Now {
+        int item, inst;
+        Range rg;
+        Grid3 grid;
+        StepConsts<T> c;
+    };
+    __shared__ Now s_now;
     __shared__ int s_last;
+    const volatile Now &now = s_now;
+    const volatile StepConsts<T> &ph = s_now.c;
+    const volatile Grid3 &grid = s_now.grid;
+    march3d_init(S);
+    Ring3 ring;
     for (;;) {
+        __syncthreads(); // everyone is done with the previous item
+        if (threadIdx.x == 0) {
+            const int w = (int)atomicAdd(counter, 1u);
+            s_now.item = w;
+            if (w < nitems) {
+                const int i = items[w].x;
+                const Inst3<T> *I = insts + i;
+                s_now.inst = i;
+                s_now.rg = ranges[i];
+                s_now.grid = Grid3(I->nb_x, I->nb_y, I->nb_z, 1);
+                s_now.c = StepConsts<T>(I->ph, I->DtDx, I->DtDy, I->DtDz, (T)I->ggm1,
+                                        (T)skip_tlo2(batch_threshold(I, skip_frac)));
+            }
+        }
         __syncthreads();
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int w = s_item;
-        if (w >= nitems) break;
-        const int2 it = items[w];
-        Inst3<T> *I = insts + it.x;
-        if (!I->active) continue;
-        const int par = I->parity;
-        const int tz = it.y % I->ntz, rem = it.y / I->ntz;
-        const int ty = rem % I->nty, ck = rem / I->nty;
-        const int i0 = 1 + ck * I->chunk;
-        const March3 geo{k3TZ * tz, k3TY<T> * ty, i0, min(i0 + I->chunk - 1, I->nb_x), I->nb_x, I->nb_y, I->nb_z,
-                         I->zs, I->zy, 1};
-        const Phys<T> ph = I->ph;
+        if (now.item >= nitems) break;
         MaxAcc acc;
-        const float tlo2 = skip_tlo2(batch_threshold(I, skip_frac)), ggm1 = I->ggm1;
-        march3d<T, kF, false, k3Warps<T>, false>(
-            S, I->rhoE[par], I->uvw[par], I->rhoE[par ^ 1], I->uvw[par ^ 1], geo, ph, I->DtDx, I->DtDy, I->DtDz,
-            [&](const Upd3<T> &o) {
-                if (!state_below(o, ggm1, tlo2))
-                    acc.add_speed(o.r, (double)speed3<T, kF>(o.r, o.u, o.v, o.w, o.E, ph));
-            });
-        const int2 rg = ranges[it.x];
-        if (publish_step<k3NT<T>>(acc, parts, w, &I->done_items, rg.y, &s_last))
-            finalize_step<k3NT<T>, T, kF>(I, parts + rg.x, rg.y, status ? status + it.x : nullptr, skip_frac);
+        {
+            const Inst3<T> *I = insts + now.inst;
+            if (!I->active) continue;
+            const int par = I->parity, y = items[now.item].y;
+            const int tz = y % I->ntz, rem = y / I->ntz;
+            const int ty = rem % I->nty, ck = rem / I->nty;
+            const int i0 = 1 + ck * now.rg.chunk;
+            const March3 geo{k3TZ * tz, k3TY<T> * ty, i0, min(i0 + now.rg.chunk - 1, I->nb_x)};
+            const bool ok = march3d<T, kF>(S, I->rhoE[par], I->uvw[par], I->rhoE[par ^ 1], I->uvw[par ^ 1], geo, grid,
+                                           ph, Tmaps3{}, ring, [&](const Upd3<T> &o) {
+                                               if (!state_below(o, ph.ggm1, ph.tlo2))
+                                                   acc.add_speed(o.r, (double)speed3<T, kF>(o.r, o.u, o.v, o.w, o.E, ph));
+                                           });
+            if (!ok) acc.err |= kErrWaitTimeout;
+        }
+        Inst3<T> *I = insts + now.inst;
+        const int first = now.rg.first, count = now.rg.count;
+        if (publish_step<k3NT<T>>(acc, parts, now.item, &I->done_items, count, &s_last))
+            finalize_step<k3NT<T>, T, kF>(I, parts + first, count, status ? status + now.inst : nullptr, skip_frac);
     }
 }
 
-// End-of-run conservation sums (compensated FP64 mass, momenta, energy) of every instance
-// over the same work items: one pass over the current state after the run's last step.
-template <int NT, class T> __device__ __forceinline__ void sum_item(const Inst2<T> *I, int y, BatchAcc &acc)
+// End-of-run conservation sums (compensated FP64 mass, momenta, energy) of every instance: one
+// pass over the current state after the run's last step. An instance's items share its
+// interior cells out evenly, kSumCells to each thread, so that their number and what they hold
+// depend on the instance alone. kSumLoads cells are loaded at a time ahead of their additions,
+// which are chains of four FP64 operations each: with one cell at a time they waited for its
+// loads (10.4 M cells FP32 in 68 us, 4 at a time 74, 8 at a time 56; 15.8 M cells 3D FP64 226 us
+// one at a time, 8 at a time 140).
+constexpr int kSumNT = 128, kSumCells = 64, kSumLoads = 8;
+
+// Where an instance's interior rows lie (3D: the rows (i, j) in order), in registers.
+template <class T> struct Rows {
+    const typename Vec2<T>::type *r;
+    const T *u;
+    int len, nj;        // cells of a row, rows per plane (1 in 2D)
+    long long n, si, sj; // rows, strides of i and j in cells
+    __device__ explicit Rows(const Inst2<T> *I)
+        : r(reinterpret_cast<const typename Vec2<T>::type *>(I->rhoE[I->parity])), u(I->uv[I->parity]), len(I->nb_y),
+          nj(1), n(I->nb_x), si(I->ys), sj(0)
+    {
+    }
+    __device__ explicit Rows(const Inst3<T> *I)
+        : r(reinterpret_cast<const typename Vec2<T>::type *>(I->rhoE[I->parity])), u(I->uvw[I->parity]), len(I->nb_z),
+          nj(I->nb_y), n((long long)I->nb_x * I->nb_y), si(I->zy), sj(I->zs)
+    {
+    }
+    // the first interior cell of row q
+    __device__ __forceinline__ long long start(unsigned q) const
+    {
+        const unsigned i = q / (unsigned)nj, j = q - i * (unsigned)nj;
+        return (1 + (long long)i) * si + (sj ? (1 + (long long)j) * sj : 0) + 1;
+    }
+};
+
+template <int NT, int D, class T, class I> __device__ __forceinline__ void sum_item(const I *in, int y, int n, BatchAcc &acc)
 {
     using V2 = typename Vec2<T>::type;
-    const int strip = y % I->nstrips, ck = y / I->nstrips;
-    const int t = threadIdx.x, j = kStripW * strip + t;
-    if (t < 1 || t > kStripW || j > I->nb_y) return;
-    const int i0 = 1 + ck * I->chunk, i1 = min(i0 + I->chunk - 1, I->nb_x);
-    const V2 *r = reinterpret_cast<const V2 *>(I->rhoE[I->parity]);
-    const V2 *u = reinterpret_cast<const V2 *>(I->uv[I->parity]);
-    for (int i = i0; i <= i1; ++i) {
-        const long long c = (long long)i * I->ys + j;
-        const V2 a = r[c], b = u[c];
-        acc.add_sums<2>(a.x, b.x, b.y, T(0), a.y);
-    }
-}
-template <int NT, class T> __device__ __forceinline__ void sum_item(const Inst3<T> *I, int y, BatchAcc &acc)
-{
-    const int tz = y % I->ntz, rem = y / I->ntz;
-    const int ty = rem % I->nty, ck = rem / I->nty;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int k = k3TZ * tz + lane, j = k3TY<T> * ty + w;
-    if (w < 1 || w > k3TY<T> || lane < 1 || lane > k3TZ || j > I->nb_y || k > I->nb_z) return;
-    const int i0 = 1 + ck * I->chunk, i1 = min(i0 + I->chunk - 1, I->nb_x);
-    const T *r = I->rhoE[I->parity], *u = I->uvw[I->parity];
-    for (int i = i0; i <= i1; ++i) {
-        const long long c = (long long)i * I->zy + (long long)j * I->zs + k;
-        acc.add_sums<3>(r[2 * c], u[3 * c], u[3 * c + 1], u[3 * c + 2], r[2 * c + 1]);
+    const Rows<T> g(in);
+    const long long total = g.n * g.len, q0 = total * y / n;
+    int left = (int)(total * (y + 1) / n - q0) - (int)threadIdx.x; // cells from this thread's on
+    unsigned row = (unsigned)((q0 + threadIdx.x) / g.len);
+    int col = (int)((q0 + threadIdx.x) - (long long)row * g.len);
+    long long base = g.start(row);
+    while (left > 0) {
+        long long c[kSumLoads];
+        int got = 0;
+#pragma unroll
+        for (int e = 0; e < kSumLoads; ++e) {
+            c[e] = base + col;
+            got += left > 0;
+            left -= NT;
+            col += NT;
+            if (col >= g.len && left > 0) {
+                do {
+                    col -= g.len;
+                    ++row;
+                } while (col >= g.len);
+                base = g.start(row);
+            }
+        }
+        V2 a[kSumLoads], b[kSumLoads];
+        T m2[kSumLoads];
+#pragma unroll
+        for (int e = 0; e < kSumLoads; ++e) {
+            const long long k = e < got ? c[e] : c[0];
+            a[e] = __ldg(g.r + k);
+            if (D == 2) {
+                b[e] = __ldg(reinterpret_cast<const V2 *>(g.u) + k);
+            } else {
+                b[e].x = __ldg(g.u + 3 * k);
+                b[e].y = __ldg(g.u + 3 * k + 1);
+                m2[e] = __ldg(g.u + 3 * k + 2);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < kSumLoads; ++e)
+            if (e < got) acc.add_sums<D>(a[e].x, b[e].x, b[e].y, D == 3 ? m2[e] : T(0), a[e].y);
     }
 }
 
-template <int NT, class T, class I>
-__global__ void __launch_bounds__(NT) batch_sums(I *insts, const int2 *items, const int2 *ranges, int nitems,
+template <int NT, int D, class T, class I>
+__global__ void __launch_bounds__(NT) batch_sums(I *insts, const int2 *items, const Range *ranges, int nitems,
                                                  unsigned *counter, ItemPart *parts, SlotStatus *status)
 {
     __shared__ int s_item;
@@ -500,10 +582,10 @@ __global__ void __launch_bounds__(NT) batch_sums(I *insts, const int2 *items, co
         const int2 it = items[w];
         I *in = insts + it.x;
         BatchAcc acc;
-        sum_item<NT, T>(in, it.y, acc);
-        const int2 rg = ranges[it.x];
-        if (publish_item<NT>(acc, parts, w, &in->sum_items, rg.y, &s_last))
-            finalize_sums<NT>(in, parts + rg.x, rg.y, status ? status + it.x : nullptr);
+        const Range rg = ranges[it.x];
+        sum_item<NT, D, T>(in, it.y, rg.sum_count, acc);
+        if (publish_item<NT>(acc, parts, rg.sum_first + it.y, &in->sum_items, rg.sum_count, &s_last))
+            finalize_sums<NT>(in, parts + rg.sum_first, rg.sum_count, status ? status + it.x : nullptr);
     }
 }
 
@@ -529,14 +611,14 @@ template <class T, int D> class BatchEngine final : public BatchBase {
 
   public:
     BatchEngine(int chunk, int capacity, cudaStream_t stream, int *rc)
-        : chunk_(chunk > 0 ? chunk : (D == 2 ? 32 : 64)), cap_(capacity)
+        : chunk_(chunk), cap_(capacity)
     {
         own_stream_ = (stream == nullptr);
         cudaError_t e = cudaSuccess;
         if (own_stream_) e = cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking);
         else stream_ = stream;
         if (e == cudaSuccess) e = cudaMalloc(&insts_, sizeof(Inst) * cap_);
-        if (e == cudaSuccess) e = cudaMalloc(&ranges_, sizeof(int2) * cap_);
+        if (e == cudaSuccess) e = cudaMalloc(&ranges_, sizeof(Range) * cap_);
         if (e == cudaSuccess) e = cudaMalloc(&counter_, 64);
         if (e == cudaSuccess) e = cudaMalloc(&scratch_bits_, 64);
         if (e == cudaSuccess) e = cudaMemset(scratch_bits_, 0, 64);
@@ -553,7 +635,7 @@ template <class T, int D> class BatchEngine final : public BatchBase {
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch2d<T, false>, kStripNT, 0);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, batch2d<T, true>, kStripNT, 0);
         } else {
-            smem_ = (int)sizeof(Smem3<T>);
+            smem_ = (int)sizeof(Tile3<T>);
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(batch3d<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_);
             if (e == cudaSuccess)
@@ -566,14 +648,11 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         blocks_ = nsm * std::max(1, std::min(occ, occ_f));
         int occ_s = 0;
         if (e == cudaSuccess) {
-            if constexpr (D == 2)
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, batch_sums<kStripNT, T, Inst>, kStripNT, 0);
-            else
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, batch_sums<k3NT<T>, T, Inst>, k3NT<T>, 0);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, batch_sums<kSumNT, D, T, Inst>, kSumNT, 0);
         }
         sum_blocks_ = nsm * std::max(1, occ_s);
         slots_.resize(cap_);
-        host_ranges_.assign(cap_, make_int2(0, 0));
+        host_ranges_.assign(cap_, Range{});
         *rc = (e == cudaSuccess) ? kOk : kErrCuda;
         if (e != cudaSuccess) set_error(kErrCuda, "batch create: %s", cudaGetErrorString(e));
     }
@@ -588,7 +667,6 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         cudaFree(ranges_);
         cudaFree(counter_);
         cudaFree(scratch_bits_);
-        cudaFree(items_);
         cudaFree(parts_);
         cudaFreeHost(status_h_);
         if (own_stream_) cudaStreamDestroy(stream_);
@@ -683,10 +761,8 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         I.steps = 0;
         I.nb_x = (int)nb_x;
         I.nb_y = (int)nb_y;
-        I.chunk = chunk_;
         I.parity = 0;
         I.active = (0.0 < s.t_end) && (0 < s.max_steps);
-        int nitems;
         if constexpr (D == 2) {
             I.ys = (long long)ys;
             I.nstrips = (int)((nb_y + kStripW - 1) / kStripW);
@@ -703,7 +779,7 @@ template <class T, int D> class BatchEngine final : public BatchBase {
                     return kErrCuda;
                 }
             }
-            nitems = I.nstrips * (int)((nb_x + chunk_ - 1) / chunk_);
+            sl.tiles = I.nstrips;
         } else {
             I.DtDz = I.dt / I.DZ;
             I.nb_z = (int)nb_z;
@@ -715,7 +791,7 @@ template <class T, int D> class BatchEngine final : public BatchBase {
                 I.rhoE[b] = sl.rhoE[b];
                 I.uvw[b] = sl.uvx[b];
             }
-            nitems = I.ntz * I.nty * (int)((nb_x + chunk_ - 1) / chunk_);
+            sl.tiles = I.ntz * I.nty;
         }
         e = cudaMemcpyAsync(insts_ + slot, &I, sizeof I, cudaMemcpyHostToDevice, stream_);
         SlotStatus st0{};
@@ -729,7 +805,6 @@ template <class T, int D> class BatchEngine final : public BatchBase {
             return kErrCuda;
         }
         sl.used = true;
-        sl.nitems = nitems;
         sl.ys = ys;
         sl.nb[0] = nb_x;
         sl.nb[1] = nb_y;
@@ -876,7 +951,7 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     struct Slot {
         bool used = false;
         T *rhoE[2] = {nullptr, nullptr}, *uvx[2] = {nullptr, nullptr};
-        int nitems = 0;
+        int tiles = 0; // strips (2D) or tiles (3D)
         size_t ys = 0, nb[3] = {0, 0, 0};
     };
 
@@ -888,7 +963,7 @@ template <class T, int D> class BatchEngine final : public BatchBase {
             s.rhoE[b] = s.uvx[b] = nullptr;
         }
         s.used = false;
-        s.nitems = 0;
+        s.tiles = 0;
     }
 
     void launch()
@@ -906,43 +981,87 @@ template <class T, int D> class BatchEngine final : public BatchBase {
 
     void launch_sums()
     {
-        if constexpr (D == 2)
-            batch_sums<kStripNT, T, Inst><<<sum_blocks_, kStripNT, 0, stream_>>>(insts_, items_, ranges_, nitems_,
-                                                                                counter_ + 1, parts_, status_d_);
-        else
-            batch_sums<k3NT<T>, T, Inst><<<sum_blocks_, k3NT<T>, 0, stream_>>>(insts_, items_, ranges_, nitems_,
-                                                                        counter_ + 1, parts_, status_d_);
+        batch_sums<kSumNT, D, T, Inst><<<sum_blocks_, kSumNT, 0, stream_>>>(insts_, sum_list_, ranges_, nsums_,
+                                                                           counter_ + 1, parts_, status_d_);
+    }
+
+    // Rows (planes) per step item, at most: the caller's, or the one with the shortest
+    // estimated step: every item costs its rows and about 3 more (halo rows, start and end), the
+    // resident blocks share them out, and at the end they wait for half an item on average. Long
+    // items suit a set that fills the GPU many times over, short ones a set of a few
+    // instances.
+    int pick_chunk() const
+    {
+        if (chunk_ > 0) return chunk_;
+        int best = 0;
+        double best_cost = 0.0;
+        for (int c : {8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256}) {
+            double work = 0.0;
+            int longest = 0;
+            for (const Slot &s : slots_) {
+                if (!s.used) continue;
+                const int n = ((int)s.nb[0] + c - 1) / c, own = ((int)s.nb[0] + n - 1) / n;
+                work += (double)s.tiles * ((double)s.nb[0] + 3.0 * n);
+                longest = std::max(longest, own);
+            }
+            const double cost = work / blocks_ + 0.5 * (longest + 3);
+            if (best == 0 || cost < best_cost) {
+                best = c;
+                best_cost = cost;
+            }
+        }
+        return best;
     }
 
     // Work list and partial slots for the instances in use; the graph of `nsteps` steps
     // followed by the conservation sums.
     int rebuild(int nsteps)
     {
-        std::vector<int2> items;
+        // step items: each instance's rows in even chunks, the instances with the longest
+        // first, so that the last items to be taken are short ones
+        const int cap = pick_chunk();
+        std::vector<int> order;
         for (int i = 0; i < cap_; ++i) {
-            if (!slots_[i].used) {
-                host_ranges_[i] = make_int2(0, 0);
-                continue;
-            }
-            host_ranges_[i] = make_int2((int)items.size(), slots_[i].nitems);
-            for (int k = 0; k < slots_[i].nitems; ++k) items.push_back(make_int2(i, k));
+            host_ranges_[i] = Range{};
+            if (!slots_[i].used) continue;
+            const int nx = (int)slots_[i].nb[0], n = (nx + cap - 1) / cap;
+            host_ranges_[i].chunk = (nx + n - 1) / n;
+            order.push_back(i);
+        }
+        std::stable_sort(order.begin(), order.end(),
+                         [&](int a, int b) { return host_ranges_[a].chunk > host_ranges_[b].chunk; });
+        std::vector<int2> items, sums;
+        for (int i : order) {
+            Range &r = host_ranges_[i];
+            const Slot &sl = slots_[i];
+            r.first = (int)items.size();
+            r.count = sl.tiles * (((int)sl.nb[0] + r.chunk - 1) / r.chunk);
+            for (int k = 0; k < r.count; ++k) items.push_back(make_int2(i, k));
+            const size_t cells = sl.nb[0] * sl.nb[1] * (D == 3 ? sl.nb[2] : 1), per = (size_t)kSumNT * kSumCells;
+            r.sum_first = (int)sums.size();
+            r.sum_count = (int)((cells + per - 1) / per);
+            for (int k = 0; k < r.sum_count; ++k) sums.push_back(make_int2(i, k));
         }
         cudaError_t e = cudaStreamSynchronize(stream_);
-        if (e == cudaSuccess && items.size() > items_cap_) {
-            cudaFree(items_);
+        const size_t most = std::max(items.size(), sums.size());
+        if (e == cudaSuccess && most > items_cap_) {
+            // one allocation: the parts, the step items, the items of the sums
             cudaFree(parts_);
-            items_ = nullptr;
             parts_ = nullptr;
-            items_cap_ = std::max(items.size(), 2 * items_cap_);
-            e = cudaMalloc(&items_, sizeof(int2) * items_cap_);
-            if (e == cudaSuccess) e = cudaMalloc(&parts_, sizeof(ItemPart) * items_cap_);
+            items_cap_ = std::max(most, 2 * items_cap_);
+            e = cudaMalloc(&parts_, (sizeof(ItemPart) + 2 * sizeof(int2)) * items_cap_);
+            items_ = reinterpret_cast<int2 *>(parts_ + items_cap_);
+            sum_list_ = items_ + items_cap_;
             if (e != cudaSuccess) items_cap_ = 0;
         }
         nitems_ = (int)items.size();
+        nsums_ = (int)sums.size();
         if (e == cudaSuccess && nitems_ > 0)
             e = cudaMemcpyAsync(items_, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, stream_);
+        if (e == cudaSuccess && nsums_ > 0)
+            e = cudaMemcpyAsync(sum_list_, sums.data(), sizeof(int2) * sums.size(), cudaMemcpyHostToDevice, stream_);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(ranges_, host_ranges_.data(), sizeof(int2) * cap_, cudaMemcpyHostToDevice, stream_);
+            e = cudaMemcpyAsync(ranges_, host_ranges_.data(), sizeof(Range) * cap_, cudaMemcpyHostToDevice, stream_);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
         if (graph_) {
             cudaGraphExecDestroy(graph_);
@@ -984,15 +1103,16 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     bool own_stream_ = false, dirty_ = true;
     cudaStream_t stream_ = nullptr;
     Inst *insts_ = nullptr;
-    int2 *ranges_ = nullptr, *items_ = nullptr;
+    Range *ranges_ = nullptr;
+    int2 *items_ = nullptr, *sum_list_ = nullptr;
     size_t items_cap_ = 0;
     ItemPart *parts_ = nullptr;
     unsigned *counter_ = nullptr;
     unsigned long long *scratch_bits_ = nullptr;
     SlotStatus *status_h_ = nullptr, *status_d_ = nullptr;
     std::vector<Slot> slots_;
-    std::vector<int2> host_ranges_;
-    int nitems_ = 0, blocks_ = 1, sum_blocks_ = 1, graph_steps_ = -1, smem_ = 0;
+    std::vector<Range> host_ranges_;
+    int nitems_ = 0, nsums_ = 0, blocks_ = 1, sum_blocks_ = 1, graph_steps_ = -1, smem_ = 0;
     cudaGraphExec_t graph_ = nullptr;
 };
 

@@ -74,14 +74,14 @@ template <class T> __global__ void __launch_bounds__(kDirectNT) direct2d(Args2<T
         const Cell2<T> P = make_cell2<T>(ur, uu, uv, uE, g.ph);
         const Cell2<T> PL = load_cell2(g, (long long)(g.xwrap ? wrap_row(i - 1, g.nb_x) : i - 1) * g.ys + j);
         const Cell2<T> PR = load_cell2(g, (long long)(g.xwrap ? wrap_row(i + 1, g.nb_x) : i + 1) * g.ys + j);
-        const Flux2<T> fx1 = face_flux(face_x(PL), face_x(P), g.ph);
-        const Flux2<T> fx2 = face_flux(face_x(P), face_x(PR), g.ph);
+        const Flux2<T> fx1 = face_flux(face_x(PL), face_x(P));
+        const Flux2<T> fx2 = face_flux(face_x(P), face_x(PR));
         const FaceIn<T> me = face_y(P);
         const FaceIn<T> lo = (j == 1) ? mirror(me) : face_y(load_cell2(g, c - 1));
         const FaceIn<T> hi = (j == g.nb_y) ? mirror(me) : face_y(load_cell2(g, c + 1));
-        const Flux2<T> fy1 = face_flux(lo, me, g.ph);
-        const Flux2<T> fy2 = face_flux(me, hi, g.ph);
-        const Upd2<T> o = update2(ur, uu, uv, uE, fx1, fx2, fy1, fy2, g.DtDx, g.DtDy, g.ph);
+        const Flux2<T> fy1 = face_flux(lo, me);
+        const Flux2<T> fy2 = face_flux(me, hi);
+        const Upd2<T> o = update2(ur, uu, uv, uE, fx1, fx2, fy1, fy2, g.DtDx, g.DtDy);
         g.rhoE_n[2 * c] = o.r;
         g.rhoE_n[2 * c + 1] = o.E;
         g.uv_n[2 * c] = o.u;

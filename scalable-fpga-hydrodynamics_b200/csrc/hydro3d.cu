@@ -9,18 +9,16 @@
 //
 // Kernels:
 //  strip3d   one CTA of W warps over a tile of rows (y) x 32 (z) columns with a one-cell
-//            halo ring, marching down `chunk` X planes: by default 9 rows on 8 warps
-//            (7 x 30 interior cells; warp 0 holds both halo rows) where tensor maps stage
-//            the planes (FP64, even NB_Z), else 8 rows on 8 warps (6 x 30). Planes arrive
-//            in a shared-memory ring by tensor-map TMA loads or per-lane cp.async (any
-//            alignment of the interleaved pairs/triples); each lane converts its cell to
-//            primitives once and per plane computes one x face (registers), one z face
-//            (flux back by warp shuffles) and one y face (shared memory, double-buffered by
-//            plane parity, one barrier per plane), then updates the plane behind it.
+//            halo ring, marching down `chunk` X planes: 9 rows on 8 warps (7 x 30 interior
+//            cells; warp 0 holds both halo rows) unless another height is set. Planes arrive
+//            in a shared-memory ring by tensor-map TMA loads (FP64, even NB_Z) or by 16-byte
+//            row copies; each lane converts its cell to primitives once and per plane
+//            computes one x face, one z face (flux back by warp shuffles) and one y face
+//            (shared memory, double-buffered by plane parity, one barrier per plane), then
+//            updates the plane behind it.
 //  direct3d  one thread per cell, the 7-point stencil loaded directly, every face
 //            evaluated from both sides like the reference.
 #include <algorithm>
-#include <type_traits>
 #include <cstring>
 #include <stdio.h>
 
@@ -35,6 +33,8 @@ template <class T> struct Args3 {
     T *Dt_next;
     Phys<T> ph;
     T DtDx, DtDy, DtDz;
+    StepConsts<T> c; // the same for the strip kernel
+    Grid3 grid;
     int nb_x, nb_y, nb_z;
     long long zs, zy;
     int chunk;
@@ -67,19 +67,19 @@ template <class T> __global__ void __launch_bounds__(128) direct3d(Args3<T> g)
         const Cell3<T> P = make_cell3<T>(ur, uu, uv, uw, uE, g.ph);
         const long long cxm = (long long)(g.xwrap ? wrap_plane(i - 1, g.nb_x) : i - 1) * g.zy + (long long)j * g.zs + k;
         const long long cxp = (long long)(g.xwrap ? wrap_plane(i + 1, g.nb_x) : i + 1) * g.zy + (long long)j * g.zs + k;
-        const Flux3<T> fx1 = face_flux3(face3_x(load_cell3(g, cxm)), face3_x(P), g.ph);
-        const Flux3<T> fx2 = face_flux3(face3_x(P), face3_x(load_cell3(g, cxp)), g.ph);
+        const Flux3<T> fx1 = face_flux3(face3_x(load_cell3(g, cxm)), face3_x(P));
+        const Flux3<T> fx2 = face_flux3(face3_x(P), face3_x(load_cell3(g, cxp)));
         const FaceIn3<T> my = face3_y(P);
         const FaceIn3<T> ylo = (j == 1) ? mirror3(my) : face3_y(load_cell3(g, c - g.zs));
         const FaceIn3<T> yhi = (j == g.nb_y) ? mirror3(my) : face3_y(load_cell3(g, c + g.zs));
-        const Flux3<T> fy1 = face_flux3(ylo, my, g.ph);
-        const Flux3<T> fy2 = face_flux3(my, yhi, g.ph);
+        const Flux3<T> fy1 = face_flux3(ylo, my);
+        const Flux3<T> fy2 = face_flux3(my, yhi);
         const FaceIn3<T> mz = face3_z(P);
         const FaceIn3<T> zlo = (k == 1) ? mirror3(mz) : face3_z(load_cell3(g, c - 1));
         const FaceIn3<T> zhi = (k == g.nb_z) ? mirror3(mz) : face3_z(load_cell3(g, c + 1));
-        const Flux3<T> fz1 = face_flux3(zlo, mz, g.ph);
-        const Flux3<T> fz2 = face_flux3(mz, zhi, g.ph);
-        const Upd3<T> o = update3(ur, uu, uv, uw, uE, fx1, fx2, fy1, fy2, fz1, fz2, g.DtDx, g.DtDy, g.DtDz, g.ph);
+        const Flux3<T> fz1 = face_flux3(zlo, mz);
+        const Flux3<T> fz2 = face_flux3(mz, zhi);
+        const Upd3<T> o = update3(ur, uu, uv, uw, uE, fx1, fx2, fy1, fy2, fz1, fz2, g.DtDx, g.DtDy, g.DtDz);
         g.rhoE_n[2 * c] = o.r;
         g.rhoE_n[2 * c + 1] = o.E;
         g.uvw_n[3 * c] = o.u;
@@ -110,59 +110,47 @@ template <class T, bool kF = false> __global__ void __launch_bounds__(k3RedoNT) 
 }
 
 // ------------------------------------------------------------------- strip kernel ---
-// kF: fused arithmetic (hydro_math.cuh). kTma: planes staged by the tensor maps tmr/tmu
-// (FP64, even NB_Z), else by per-lane cp.async. W: warps per block. Tile rows with halo:
-// W, or W + 1 with kPair (tensor maps, W = 8: warp 0 holds both halo rows).
-template <class T, bool kF, bool kTma, int W, bool kPair = false>
-__global__ void __launch_bounds__(32 * W, min_blocks3<T>(W))
+// kF: fused arithmetic (hydro_math.cuh). SM: the tile (rows, warps) and its staging, by the
+// tensor maps tmr/tmu (FP64, even NB_Z) or by row copies.
+template <class T, bool kF, class SM>
+__global__ void __launch_bounds__(32 * SM::W, min_blocks3<T>(SM::W))
     strip3d(const __grid_constant__ CUtensorMap tmr, const __grid_constant__ CUtensorMap tmu, Args3<T> g)
 {
-    static_assert(!kPair || (kTma && W == 8), "the W+1-row tile is built for tensor maps and 8 warps");
-    using SM = std::conditional_t<kPair, Smem3P<T>, Smem3<T, W>>;
-    constexpr int kRows = kPair ? W + 1 : W;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     SM &S = *reinterpret_cast<SM *>(smem_raw);
-    if constexpr (kTma) {
-        if (threadIdx.x == 0) {
-            prefetch_tensormap(&tmr);
-            prefetch_tensormap(&tmu);
-        }
-        march3d_init(S);
+    if (SM::kTma && threadIdx.x == 0) {
+        prefetch_tensormap(&tmr);
+        prefetch_tensormap(&tmu);
     }
+    march3d_init(S);
     const int i0 = 1 + g.chunk * (int)blockIdx.z;
-    const March3 geo{k3TZ * (int)blockIdx.x, (kRows - 2) * (int)blockIdx.y, i0, min(i0 + g.chunk - 1, g.nb_x),
-                     g.nb_x, g.nb_y, g.nb_z, g.zs, g.zy, g.xwrap};
+    const March3 geo{k3TZ * (int)blockIdx.x, (SM::R - 2) * (int)blockIdx.y, i0, min(i0 + g.chunk - 1, g.nb_x)};
     StepAcc acc;
     const SkipLimits lim = skip_limits(g.scr, g.key);
     const float tlo2 = skip_tlo2(lim.f), ggm1 = g.ggm1;
-    const Phys<T> ph = g.ph;
-    auto sink = [&](const Upd3<T> &o) {
-        acc.add_mass(o.r);
-        if (!state_below(o, ggm1, tlo2))
-            acc.add_speed(o.r, speed3<T, kF>(o.r, o.u, o.v, o.w, o.E, ph));
-    };
-    bool ok;
-    if constexpr (kPair)
-        ok = march3d<T, kF>(S, g.rhoE_n, g.uvw_n, geo, ph, g.DtDx, g.DtDy, g.DtDz, sink, Tmaps3{&tmr, &tmu});
-    else
-        ok = march3d<T, kF, kTma, W>(S, g.rhoE, g.uvw, g.rhoE_n, g.uvw_n, geo, ph, g.DtDx, g.DtDy, g.DtDz, sink,
-                                     Tmaps3{&tmr, &tmu});
+    // (copies: used through references to the parameters, the FP32 forms spilled)
+    const Grid3 grid = g.grid;
+    const StepConsts<T> c = g.c;
+    Ring3 ring;
+    const bool ok = march3d<T, kF>(S, g.rhoE, g.uvw, g.rhoE_n, g.uvw_n, geo, grid, c, Tmaps3{&tmr, &tmu}, ring, [&](const Upd3<T> &o) {
+                                       acc.add_mass(o.r);
+                                       if (!state_below(o, ggm1, tlo2))
+                                           acc.add_speed(o.r, speed3<T, kF>(o.r, o.u, o.v, o.w, o.E, c));
+                                   });
     if (!ok) acc.err |= kErrWaitTimeout;
-    step_epilogue<32 * W, T>(acc, g.scr, g.partials, gridDim.x * gridDim.y * gridDim.z,
-                             blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), g.ph.C_min, g.Dt_next,
-                             g.status, g.seq, (double)lim.hist, g.key);
+    step_epilogue<32 * SM::W, T>(acc, g.scr, g.partials, gridDim.x * gridDim.y * gridDim.z,
+                                 blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), g.ph.C_min, g.Dt_next,
+                                 g.status, g.seq, (double)lim.hist, g.key);
 }
 
-// Tile heights (rows with halo) the plain 3D step is built for: FP64 8, 9 (8 warps, warp 0
-// holding both halo rows; tensor-map staging only), 12 and 16; FP32 8 and 16. The
-// tensor-map staging is built for FP64 only.
+// Tile heights (rows with halo) the plain 3D step is built for: 9 (on 8 warps), 8, 16 and in
+// FP64 12. 9 is the built-in one: no warp holds a halo row only (512^3 FP64 strict 37.2 against
+// 35.3 GCell/s for 8 rows).
+constexpr int kRows3 = 9;
 template <class T> constexpr bool tile3_built(int rows)
 {
-    return sizeof(T) == 8 ? (rows == 8 || rows == 9 || rows == 12 || rows == 16) : (rows == 8 || rows == 16);
+    return rows == 8 || rows == 9 || rows == 16 || (sizeof(T) == 8 && rows == 12);
 }
-// The built-in tile height: 9 rows where tensor maps stage the planes (FP64: 37.2 against
-// 35.3 GCell/s strict at 512^3 for 8 rows), else 8.
-template <class T> int default_rows3(bool tma) { return (sizeof(T) == 8 && tma) ? 9 : k3Warps<T>; }
 
 // A built form of the step: the kernel, its threads and its dynamic shared memory.
 template <class T> struct Form3 {
@@ -170,33 +158,25 @@ template <class T> struct Form3 {
     int threads = 0, smem = 0;
 };
 
-template <class T, int W, bool kPair = false> Form3<T> strip3d_form(bool fused, bool tma)
+template <class T, class SM> Form3<T> strip3d_form(bool fused)
 {
-    Form3<T> f;
-    f.threads = 32 * W;
-    if constexpr (kPair) {
-        f.kern = fused ? strip3d<T, true, true, W, true> : strip3d<T, false, true, W, true>;
-        f.smem = (int)sizeof(Smem3P<T>);
-    } else {
-        if constexpr (sizeof(T) == 8)
-            f.kern = fused ? (tma ? strip3d<T, true, true, W> : strip3d<T, true, false, W>)
-                           : (tma ? strip3d<T, false, true, W> : strip3d<T, false, false, W>);
-        else
-            f.kern = fused ? strip3d<T, true, false, W> : strip3d<T, false, false, W>;
-        f.smem = (int)sizeof(Smem3<T, W>);
-    }
-    return f;
+    return Form3<T>{fused ? strip3d<T, true, SM> : strip3d<T, false, SM>, 32 * SM::W, (int)sizeof(SM)};
 }
-
-// The form of a tile height: 9 rows run on 8 warps (FP64 tensor maps only), others on one
-// warp per row.
-template <class T> Form3<T> form3(int rows, bool fused, bool tma)
+// (tensor maps are built for FP64 only, the staging value by value for the built-in tile)
+template <class T, int W, bool kPair> Form3<T> strip3d_form(bool fused, Stage3 stage)
 {
-    if constexpr (sizeof(T) == 8) {
-        if (rows == 9) return strip3d_form<T, 8, true>(fused, true);
-        if (rows == 12) return strip3d_form<T, 12>(fused, tma);
-    }
-    return rows == 8 ? strip3d_form<T, 8>(fused, tma) : strip3d_form<T, 16>(fused, tma);
+    if constexpr (sizeof(T) == 8)
+        if (stage == Stage3::Tma) return strip3d_form<T, Smem3<T, W, kPair, Stage3::Tma>>(fused);
+    return strip3d_form<T, Smem3<T, W, kPair, Stage3::Rows>>(fused);
+}
+template <class T> Form3<T> form3(int rows, bool fused, Stage3 stage)
+{
+    if (stage == Stage3::Values) return strip3d_form<T, Smem3<T, 8, true, Stage3::Values>>(fused);
+    if constexpr (sizeof(T) == 8)
+        if (rows == 12) return strip3d_form<T, 12, false>(fused, stage);
+    if (rows == 8) return strip3d_form<T, 8, false>(fused, stage);
+    if (rows == 16) return strip3d_form<T, 16, false>(fused, stage);
+    return strip3d_form<T, 8, true>(fused, stage);
 }
 
 // ------------------------------------------------------------- initial condition ---
@@ -306,12 +286,14 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
     Args3<T> g;
     g.rhoE = rhoE; g.uvw = uvw; g.rhoE_n = rhoE_next; g.uvw_n = uvw_next; g.Dt_next = Dt_next;
     g.ph = ph; g.DtDx = DtDx; g.DtDy = DtDy; g.DtDz = DtDz;
+    g.c = StepConsts<T>(ph, DtDx, DtDy, DtDz);
     g.nb_x = (int)nb_x; g.nb_y = (int)nb_y; g.nb_z = (int)nb_z;
     g.zs = (long long)nb_z + 2; g.zy = (long long)(nb_y + 2) * g.zs;
     g.scr = ctx->scr; g.status = ctx->status_d; g.seq = ++ctx->seq;
     g.key = problem_key(Dt_next, nb_x, nb_y, nb_z, sizeof(T), ph);
     g.ggm1 = skip_ggm1(ph.gamma, ph.gm1);
     g.xwrap = xwrap ? 1 : 0;
+    g.grid = Grid3((int)nb_x, (int)nb_y, (int)nb_z, g.xwrap);
 
     const bool use_strip = which != Kernel::Direct;
     unsigned nblocks;
@@ -320,12 +302,13 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
         // (hydro_set_launch_shape), else the built-in one
         const LaunchShape shape = launch_shape(3, sizeof(T));
         // planes by tensor maps where the rows of both arrays are 16-byte pitched (FP64
-        // with even NB_Z; the tile's kbase is a multiple of 30, so even) and the arrays
-        // 16-byte aligned; by per-lane copies otherwise
-        bool tma = sizeof(T) == 8 && (nb_z + 2) % 2 == 0 && aligned16(rhoE) && aligned16(uvw);
-        // tile rows with halo; the 9-row tile needs the tensor maps (else 8 rows)
-        int rows = (shape.warps > 0 && tile3_built<T>(shape.warps)) ? shape.warps : default_rows3<T>(tma);
-        if (rows == 9 && !tma) rows = 8;
+        // with even NB_Z; the tile's kbase is a multiple of 30, so even), by row copies
+        // elsewhere; both need 16-byte aligned arrays
+        const bool wide = aligned16(rhoE) && aligned16(uvw) && aligned16(rhoE_next) && aligned16(uvw_next);
+        const bool tma = sizeof(T) == 8 && (nb_z + 2) % 2 == 0 && wide;
+        const Stage3 stage = tma ? Stage3::Tma : wide ? Stage3::Rows : Stage3::Values;
+        // tile rows with halo
+        const int rows = (wide && shape.warps > 0 && tile3_built<T>(shape.warps)) ? shape.warps : kRows3;
         const int W = rows == 9 ? 8 : rows; // warps per block
         const int nz = (int)((nb_z + k3TZ - 1) / k3TZ), ny = (int)((nb_y + (rows - 2) - 1) / (rows - 2));
         if (ny > 65535) {
@@ -333,7 +316,7 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
             return kErrArg;
         }
         // planes per block: at most the cap (the tuned value when one is set, else 256)
-        const Form3<T> form = form3<T>(rows, fused, tma);
+        const Form3<T> form = form3<T>(rows, fused, stage);
         int per_sm = 1;
         cudaError_t ea = blocks_per_sm(reinterpret_cast<const void *>(form.kern), form.threads, form.smem, &per_sm);
         if (ea != cudaSuccess) {
@@ -355,11 +338,10 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
         std::memset(&tmu, 0, sizeof tmu);
         if (tma) {
             const uint64_t zs = nb_z + 2, ys = nb_y + 2, xs = nb_x + 2;
-            tma = encode_tmap_3d(&tmr, tmap_type3<T>(), rhoE, 2 * zs, ys, xs, 2 * zs * sizeof(T), 2 * zs * ys * sizeof(T),
-                                 64, (uint32_t)rows, 1) &&
-                  encode_tmap_3d(&tmu, tmap_type3<T>(), uvw, 3 * zs, ys, xs, 3 * zs * sizeof(T), 3 * zs * ys * sizeof(T),
-                                 96, (uint32_t)rows, 1);
-            if (!tma) {
+            if (!encode_tmap_3d(&tmr, tmap_type3<T>(), rhoE, 2 * zs, ys, xs, 2 * zs * sizeof(T), 2 * zs * ys * sizeof(T),
+                                64, (uint32_t)rows, 1) ||
+                !encode_tmap_3d(&tmu, tmap_type3<T>(), uvw, 3 * zs, ys, xs, 3 * zs * sizeof(T), 3 * zs * ys * sizeof(T),
+                                96, (uint32_t)rows, 1)) {
                 set_error(kErrCuda, "step3d: tensor maps rejected");
                 return kErrCuda;
             }

@@ -222,6 +222,24 @@ template <class T> struct Phys {
     }
 };
 
+// The constants and the step's Dt / DX ... together, as the marches read them: where they lie in
+// the kernel's parameters (constant bank) every use is an operand. The persistent batch kernels
+// hold the instance's in shared memory and read them as volatile, one load per use: in
+// registers they cost 20 to 30 of the 128 and the loops spilled.
+template <class T> struct StepConsts {
+    T gamma, gm1, divgamma, K, iK;
+    bool odd;
+    T DtDx, DtDy, DtDz;
+    T ggm1, tlo2; // of the signal-speed skip (batch)
+
+    StepConsts() = default;
+    __host__ __device__ StepConsts(const Phys<T> &ph, T x, T y, T z, T g = T(0), T lo2 = T(0))
+        : gamma(ph.gamma), gm1(ph.gm1), divgamma(ph.divgamma), K(ph.K), iK(ph.iK), odd(ph.odd), DtDx(x), DtDy(y), DtDz(z),
+          ggm1(g), tlo2(lo2)
+    {
+    }
+};
+
 // A cell seen by the face flux: everything compute_fluxes needs from one side
 // (hydro2d/kernel.cxx:74-118), with the normal velocity and normal/tangential momenta
 // already routed for the face direction.
@@ -269,8 +287,8 @@ template <class T> struct Cell2 {
 // (E/rho - temp/2, and the 1/2 of the kinetic energy taken off the product r temp instead of
 // off r): the same rounding of the same value, one operation less each. A product so small
 // that 1/2 of it would round lies far below the ulp of the sum it enters.
-template <class T, bool kF = false>
-__device__ __forceinline__ Cell2<T> cell2_fast(T ur, T uu, T uv, T uE, const Phys<T> &ph, bool &bad)
+template <class T, bool kF = false, class PH>
+__device__ __forceinline__ Cell2<T> cell2_fast(T ur, T uu, T uv, T uE, const PH &ph, bool &bad)
 {
     using A = Ar<T>;
     using F = Fu<T>;
@@ -302,11 +320,11 @@ __device__ __forceinline__ Cell2<T> cell2_fast(T ur, T uu, T uv, T uE, const Phy
     return c;
 }
 
-template <class T, bool kF = false>
-__device__ __forceinline__ Cell2<T> make_cell2_checked(T ur, T uu, T uv, T uE, const Phys<T> &ph);
+template <class T, bool kF = false, class PH>
+__device__ __forceinline__ Cell2<T> make_cell2_checked(T ur, T uu, T uv, T uE, const PH &ph);
 
-template <class T, bool kF = false>
-__device__ __forceinline__ Cell2<T> make_cell2(T ur, T uu, T uv, T uE, const Phys<T> &ph)
+template <class T, bool kF = false, class PH>
+__device__ __forceinline__ Cell2<T> make_cell2(T ur, T uu, T uv, T uE, const PH &ph)
 {
     bool bad;
     Cell2<T> c = cell2_fast<T, kF>(ur, uu, uv, uE, ph, bad);
@@ -315,8 +333,8 @@ __device__ __forceinline__ Cell2<T> make_cell2(T ur, T uu, T uv, T uE, const Phy
 }
 
 // The per-cell conversion with the range checks inside the chain (both arithmetics).
-template <class T, bool kF>
-__device__ __forceinline__ Cell2<T> make_cell2_checked(T ur, T uu, T uv, T uE, const Phys<T> &ph)
+template <class T, bool kF, class PH>
+__device__ __forceinline__ Cell2<T> make_cell2_checked(T ur, T uu, T uv, T uE, const PH &ph)
 {
     using A = Ar<T>;
     Cell2<T> c;
@@ -380,7 +398,7 @@ template <class T> __device__ __forceinline__ FaceIn<T> mirror(const FaceIn<T> &
 
 // compute_fluxes, hydro2d/kernel.cxx:74-118, from cached per-cell quantities.
 template <class T, bool kF = false>
-__device__ __forceinline__ Flux2<T> face_flux(const FaceIn<T> &L, const FaceIn<T> &R, const Phys<T> &ph)
+__device__ __forceinline__ Flux2<T> face_flux(const FaceIn<T> &L, const FaceIn<T> &R)
 {
     using A = Ar<T>;
     // std::max(a_left, a_right) takes a_right iff a_left < a_right; K < 0 flips the sign of
@@ -427,8 +445,7 @@ template <class T> struct Upd2 {
 
 template <class T, bool kF = false>
 __device__ __forceinline__ Upd2<T> update2(T ur, T uu, T uv, T uE, const Flux2<T> &fx_lo, const Flux2<T> &fx_hi,
-                                           const Flux2<T> &fy_lo, const Flux2<T> &fy_hi, T DtDx, T DtDy,
-                                           const Phys<T> &ph)
+                                           const Flux2<T> &fy_lo, const Flux2<T> &fy_hi, T DtDx, T DtDy)
 {
     using A = Ar<T>;
     if constexpr (kF) {
@@ -459,7 +476,7 @@ __device__ __forceinline__ Upd2<T> update2(T ur, T uu, T uv, T uE, const Flux2<T
 }
 
 // Signal speed c_s + |u| of a 2D state, hydro2d/kernel.cxx:287-309.
-template <class T, bool kF = false> __device__ __forceinline__ T speed2(T r, T ru, T rv, T E, const Phys<T> &ph)
+template <class T, bool kF = false, class PH> __device__ __forceinline__ T speed2(T r, T ru, T rv, T E, const PH &ph)
 {
     using A = Ar<T>;
     if constexpr (kF) {
@@ -511,13 +528,14 @@ __device__ __forceinline__ bool speed_below(double r, double E, double m2, doubl
                     (unsigned)__double2hiint(m2) < m_hi;
     return in && (ggm1 * E * r + m2) * (2.0 * (1.0 + 1.0 / 4096.0)) < tlo2 * (r * r);
 }
-// The skip test of a new 2D / 3D state in the state's own precision.
-template <class T> __device__ __forceinline__ bool state_below(const Upd2<T> &o, float ggm1, float tlo2)
+// The skip test of a new 2D / 3D state in the state's own precision (S: float, or the constants
+// already in it).
+template <class T, class S> __device__ __forceinline__ bool state_below(const Upd2<T> &o, S ggm1, S tlo2)
 {
     return speed_below(o.r, o.E, o.u * o.u + o.v * o.v, (T)ggm1, (T)tlo2);
 }
 template <class T> struct Upd3;
-template <class T> __device__ __forceinline__ bool state_below(const Upd3<T> &o, float ggm1, float tlo2)
+template <class T, class S> __device__ __forceinline__ bool state_below(const Upd3<T> &o, S ggm1, S tlo2)
 {
     return speed_below(o.r, o.E, o.u * o.u + o.v * o.v + o.w * o.w, (T)ggm1, (T)tlo2);
 }
@@ -542,8 +560,8 @@ template <class T> struct Cell3 {
 };
 
 // As cell2_fast.
-template <class T, bool kF = false>
-__device__ __forceinline__ Cell3<T> cell3_fast(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph, bool &bad)
+template <class T, bool kF = false, class PH>
+__device__ __forceinline__ Cell3<T> cell3_fast(T ur, T uu, T uv, T uw, T uE, const PH &ph, bool &bad)
 {
     using A = Ar<T>;
     using F = Fu<T>;
@@ -588,11 +606,11 @@ __device__ __forceinline__ Cell3<T> cell3_fast(T ur, T uu, T uv, T uw, T uE, con
     return c;
 }
 
-template <class T, bool kF = false>
-__device__ __forceinline__ Cell3<T> make_cell3_checked(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph);
+template <class T, bool kF = false, class PH>
+__device__ __forceinline__ Cell3<T> make_cell3_checked(T ur, T uu, T uv, T uw, T uE, const PH &ph);
 
-template <class T, bool kF = false>
-__device__ __forceinline__ Cell3<T> make_cell3(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph)
+template <class T, bool kF = false, class PH>
+__device__ __forceinline__ Cell3<T> make_cell3(T ur, T uu, T uv, T uw, T uE, const PH &ph)
 {
     bool bad;
     Cell3<T> c = cell3_fast<T, kF>(ur, uu, uv, uw, uE, ph, bad);
@@ -601,8 +619,8 @@ __device__ __forceinline__ Cell3<T> make_cell3(T ur, T uu, T uv, T uw, T uE, con
 }
 
 // The per-cell conversion with the range checks inside the chain (both arithmetics).
-template <class T, bool kF>
-__device__ __forceinline__ Cell3<T> make_cell3_checked(T ur, T uu, T uv, T uw, T uE, const Phys<T> &ph)
+template <class T, bool kF, class PH>
+__device__ __forceinline__ Cell3<T> make_cell3_checked(T ur, T uu, T uv, T uw, T uE, const PH &ph)
 {
     using A = Ar<T>;
     Cell3<T> c;
@@ -674,7 +692,7 @@ template <class T> __device__ __forceinline__ FaceIn3<T> mirror3(const FaceIn3<T
 
 // compute_fluxes, hydro3d/kernel.cxx:79-130
 template <class T, bool kF = false>
-__device__ __forceinline__ Flux3<T> face_flux3(const FaceIn3<T> &L, const FaceIn3<T> &R, const Phys<T> &ph)
+__device__ __forceinline__ Flux3<T> face_flux3(const FaceIn3<T> &L, const FaceIn3<T> &R)
 {
     using A = Ar<T>;
     const bool right = A::abs(L.Ka) < A::abs(R.Ka);
@@ -719,8 +737,7 @@ template <class T> struct Upd3 {
 template <class T, bool kF = false>
 __device__ __forceinline__ Upd3<T> update3(T ur, T uu, T uv, T uw, T uE, const Flux3<T> &fx_lo,
                                            const Flux3<T> &fx_hi, const Flux3<T> &fy_lo, const Flux3<T> &fy_hi,
-                                           const Flux3<T> &fz_lo, const Flux3<T> &fz_hi, T DtDx, T DtDy, T DtDz,
-                                           const Phys<T> &ph)
+                                           const Flux3<T> &fz_lo, const Flux3<T> &fz_hi, T DtDx, T DtDy, T DtDz)
 {
     using A = Ar<T>;
     if constexpr (kF) {
@@ -765,8 +782,8 @@ __device__ __forceinline__ Upd3<T> update3(T ur, T uu, T uv, T uw, T uE, const F
 }
 
 // Signal speed c_s + |u| of a 3D state, hydro3d/kernel.cxx:367-390.
-template <class T, bool kF = false>
-__device__ __forceinline__ T speed3(T r, T ru, T rv, T rw, T E, const Phys<T> &ph)
+template <class T, bool kF = false, class PH>
+__device__ __forceinline__ T speed3(T r, T ru, T rv, T rw, T E, const PH &ph)
 {
     using A = Ar<T>;
     if constexpr (kF) {

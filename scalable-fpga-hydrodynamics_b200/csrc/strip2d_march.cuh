@@ -148,7 +148,7 @@ __device__ __forceinline__ bool march2d_tma(Smem2<T> &S, const CUtensorMap *tmr,
             if (j == 0) L = mirror(R);       // wall at j = 1/2
             if (j == g.nb_y) R = mirror(me); // wall at j = NB_Y + 1/2
         }
-        return face_flux<T, kF>(L, R, ph);
+        return face_flux<T, kF>(L, R);
     };
     if (kEdge && dead_warp) {
         // (thread 0, which issues the row loads, is in warp 0: never dead)
@@ -168,7 +168,7 @@ __device__ __forceinline__ bool march2d_tma(Smem2<T> &S, const CUtensorMap *tmr,
             const Cell2<T> P = make_cell2<T, kF>(a.x, b.x, b.y, a.y, ph);
             if (m == 1) {
                 publish(m, P);
-                fxlo = face_flux<T, kF>(face_x(Pm), face_x(P), ph);
+                fxlo = face_flux<T, kF>(face_x(Pm), face_x(P));
             }
             __syncthreads(); // stage consumed by every lane; row 1's inputs published
             if (S.abort) {
@@ -186,7 +186,7 @@ __device__ __forceinline__ bool march2d_tma(Smem2<T> &S, const CUtensorMap *tmr,
                 load(m, a, b);
                 const Flux2<T> fyr = yface(m);
                 const Cell2<T> P = make_cell2<T, kF>(a.x, b.x, b.y, a.y, ph);
-                const Flux2<T> fxhi = face_flux<T, kF>(face_x(Pm), face_x(P), ph);
+                const Flux2<T> fxhi = face_flux<T, kF>(face_x(Pm), face_x(P));
                 // row m-1's right face for the next lane (its left face), double-buffered
                 // by row parity: the buffer of row m-3 was last read before the previous
                 // barrier
@@ -203,7 +203,7 @@ __device__ __forceinline__ bool march2d_tma(Smem2<T> &S, const CUtensorMap *tmr,
                     // row m-1's left face is lane t-1's right face of that row
                     const V2 f0 = S.xF[(m - 1) & 1][0][t], f1 = S.xF[(m - 1) & 1][1][t];
                     const Flux2<T> fyl{f0.x, f0.y, f1.x, f1.y};
-                    const Upd2<T> o = update2<T, kF>(Ur, Uu, Uv, UE, fxlo, fxhi, fyl, fyr, DtDx, DtDy, ph);
+                    const Upd2<T> o = update2<T, kF>(Ur, Uu, Uv, UE, fxlo, fxhi, fyl, fyr, DtDx, DtDy);
                     const long long c = (long long)(g.i0 + m - 2) * g.ys + j;
                     reinterpret_cast<V2 *>(rhoE_n)[c] = mk2<T>(o.r, o.E);
                     reinterpret_cast<V2 *>(uv_n)[c] = mk2<T>(o.u, o.v);
@@ -296,12 +296,12 @@ __device__ __forceinline__ bool march2d_lane(Smem2<T> &S, const March2 &g, T *rh
 
         if (m >= 1) {
             // x face (row n-1 | row n) of this column; then the update of row n-1
-            const Flux2<T> fxhi = face_flux<T, kF>(face_x(Pm), face_x(P), ph);
+            const Flux2<T> fxhi = face_flux<T, kF>(face_x(Pm), face_x(P));
             if (m >= 2 && interior) {
                 // row n-1's left face is lane t-1's right face of that row
                 const V2 f0 = S.xF[(m - 1) & 1][0][t], f1 = S.xF[(m - 1) & 1][1][t];
                 const Flux2<T> fyl{f0.x, f0.y, f1.x, f1.y};
-                const Upd2<T> o = update2<T, kF>(Ur, Uu, Uv, UE, fxlo, fxhi, fyl, fyr, DtDx, DtDy, ph);
+                const Upd2<T> o = update2<T, kF>(Ur, Uu, Uv, UE, fxlo, fxhi, fyl, fyr, DtDx, DtDy);
                 const long long c = (long long)(g.i0 + m - 2) * g.ys + j;
                 reinterpret_cast<V2 *>(rhoE_n)[c] = mk2<T>(o.r, o.E);
                 reinterpret_cast<V2 *>(uv_n)[c] = mk2<T>(o.u, o.v);
@@ -320,7 +320,7 @@ __device__ __forceinline__ bool march2d_lane(Smem2<T> &S, const March2 &g, T *rh
                 if (j == 0) L = mirror(R);       // wall at j = 1/2
                 if (j == g.nb_y) R = mirror(me); // wall at j = NB_Y + 1/2
             }
-            fyr = face_flux<T, kF>(L, R, ph);
+            fyr = face_flux<T, kF>(L, R);
             S.xF[m & 1][0][t + 1] = mk2<T>(fyr.r, fyr.n);
             S.xF[m & 1][1][t + 1] = mk2<T>(fyr.t, fyr.E);
         }
