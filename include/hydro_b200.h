@@ -203,8 +203,8 @@ unsigned hydro2d_noalloc_launch_shape(size_t NB_X, size_t NB_Y, int strip, int s
  *  chunk: the most rows (2D) or planes (3D) one block marches (built-in 256); blocks take
  *    fewer on grids too small to fill the GPU with that many (sized from the grid and the
  *    SM count);
- *  blocks_per_sm: 2D only, the resident blocks per SM the kernel's registers are budgeted
- *    for (4, or 5 in FP64 / 8 in FP32; built-in 4).
+ *  blocks_per_sm: 2D only, the register budget of the kernel: 4, the built-in one (4
+ *    resident blocks per SM in FP64, 7 in FP32), or 5 in FP64 / 8 in FP32.
  * Process-wide; the results do not depend on the shape. No counterpart in the reference,
  * whose single-task kernel has no launch shape. */
 int hydro_set_launch_shape(int dim, int precision_bytes, int warps, int chunk, int blocks_per_sm);

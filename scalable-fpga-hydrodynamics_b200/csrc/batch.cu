@@ -6,10 +6,10 @@
 // Each instance keeps the plain path's arithmetic: the same strip march
 // (strip2d_march.cuh / strip3d_march.cuh), so an instance's state after n batched steps
 // is bit-identical to n plain steps in the same precision. 2D instances keep the pair
-// layout with rows padded to 16 bytes (TMA-fed); 3D instances keep the reference's
+// layout with rows padded to 16 bytes; 3D instances keep the reference's
 // pair/triple layout (row copies). Work is a flat list of (instance, tile x chunk)
-// items; persistent blocks take items from an atomic counter. Every item writes its max
-// signal speed and error bits to its own slot; the item that completes an instance's
+// items; persistent blocks take one item each by their number and more from an atomic counter.
+// Every item writes its max signal speed and error bits to its own slot; the item that completes an instance's
 // step (ticket per instance) merges that instance's slots -- the result depends neither
 // on which block ran which item nor on the other instances in the batch -- and advances
 // the instance on the device:
@@ -37,7 +37,6 @@ namespace hydro {
 constexpr int kSums = 5; // rho, rho u, rho v, rho w (0 in 2D), E
 
 template <class T> struct alignas(128) Inst2 {
-    CUtensorMap tm[2][2]; // [buffer][0: (rho, E), 1: (rho u, rho v)]
     T *rhoE[2], *uv[2];
     Phys<T> ph;
     T DX, DY, dt, DtDx, DtDy;
@@ -374,6 +373,16 @@ __device__ __forceinline__ bool publish_item(BatchAcc &acc, ItemPart *parts, int
     return last;
 }
 
+// The item at hand, its instance's grid and constants, in shared memory: read again where they
+// are needed. Held in registers through the march they cost about 30 of its 128 in 3D FP64, and
+// it spilled: 8 steps of 15.8 M cells took 6.6 ms, so 4.7 ms (5.2 ms with the former march).
+template <class T, class Grid> struct Now {
+    int item, inst;
+    Range rg;
+    Grid grid;
+    StepConsts<T> c;
+};
+
 // resident blocks per SM the register budget of the 2D step aims at
 template <class T> struct Batch2dOcc { static constexpr int value = sizeof(T) == 4 ? 6 : 4; };
 
@@ -384,39 +393,51 @@ __global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<
                                                       SlotStatus *status, double skip_frac)
 {
     __shared__ Smem2<T> S;
-    __shared__ int s_item;
+    __shared__ Now<T, Grid2> s_now;
     __shared__ int s_last;
-    march2d_init(S);
-    unsigned ld = 0;
+    const volatile Now<T, Grid2> &now = s_now;
+    int next = (int)blockIdx.x; // thread 0: the item to take
     for (;;) {
-        __syncthreads(); // everyone has read s_item / finished the previous item
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int w = s_item;
-        if (w >= nitems) break;
-        const int2 it = items[w];
-        Inst2<T> *I = insts + it.x;
-        if (!I->active) continue;
-        const Range rg = ranges[it.x];
-        const int par = I->parity;
-        const int strip = it.y % I->nstrips, ck = it.y / I->nstrips;
-        const int i0 = 1 + ck * rg.chunk;
-        const March2 geo{kStripW * strip, i0, min(i0 + rg.chunk - 1, I->nb_x), I->nb_x, I->nb_y, I->ys, 1};
-        const Phys<T> ph = I->ph;
+        __syncthreads(); // everyone is done with the previous item
         if (threadIdx.x == 0) {
-            prefetch_tensormap(&I->tm[par][0]);
-            prefetch_tensormap(&I->tm[par][1]);
+            const int w = next;
+            s_now.item = w;
+            if (w < nitems) {
+                next = (int)(gridDim.x + atomicAdd(counter, 1u)); // (looked at behind this item's march)
+                const int i = items[w].x;
+                const Inst2<T> *I = insts + i;
+                s_now.inst = i;
+                s_now.rg = ranges[i];
+                s_now.grid = Grid2{I->nb_x, I->nb_y, 1, I->ys};
+                s_now.c = StepConsts<T>(I->ph, I->DtDx, I->DtDy, T(0), (T)I->ggm1,
+                                        (T)skip_tlo2(batch_threshold(I, skip_frac)));
+            }
         }
+        __syncthreads();
+        if (now.item >= nitems) break;
         MaxAcc acc;
-        const float tlo2 = skip_tlo2(batch_threshold(I, skip_frac)), ggm1 = I->ggm1;
-        const bool ok = march2d<T, true, kF>(S, &I->tm[par][0], &I->tm[par][1], geo, I->rhoE[par ^ 1], I->uv[par ^ 1], ph,
-                                   I->DtDx, I->DtDy, ld, [&](const Upd2<T> &o) {
-                                       if (!state_below(o, ggm1, tlo2))
-                                           acc.add_speed(o.r, (double)speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
-                                   });
-        if (!ok) acc.err |= kErrWaitTimeout;
-        if (publish_step<kStripNT>(acc, parts, w, &I->done_items, rg.count, &s_last))
-            finalize_step<kStripNT, T, kF>(I, parts + rg.first, rg.count, status ? status + it.x : nullptr, skip_frac);
+        {
+            const Inst2<T> *I = insts + now.inst;
+            if (!I->active) continue;
+            const int par = I->parity, y = items[now.item].y;
+            const int strip = y % I->nstrips, ck = y / I->nstrips;
+            const int i0 = 1 + ck * now.rg.chunk;
+            // (the constants stay in shared memory, the grid is copied: 24 instances of 10.4 M cells,
+            // 10 steps FP32 1183 us fused and 1184 strict, FP64 1734 strict; all in shared memory
+            // 1228 fused, constants copied 1230 FP32 strict and 1739 FP64)
+            const volatile StepConsts<T> &ph = s_now.c;
+            const Grid2 grid = s_now.grid;
+            const March2 geo{kStripW * strip, i0, min(i0 + now.rg.chunk - 1, I->nb_x)};
+            march2d<T, kF>(S, I->rhoE[par], I->uv[par], I->rhoE[par ^ 1], I->uv[par ^ 1], geo, grid, ph,
+                           [&](const Upd2<T> &o) {
+                               if (!state_below(o, ph.ggm1, ph.tlo2))
+                                   acc.add_speed(o.r, (double)speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
+                           });
+        }
+        Inst2<T> *I = insts + now.inst;
+        const int first = now.rg.first, count = now.rg.count;
+        if (publish_step<kStripNT>(acc, parts, now.item, &I->done_items, count, &s_last))
+            finalize_step<kStripNT, T, kF>(I, parts + first, count, status ? status + now.inst : nullptr, skip_frac);
     }
 }
 
@@ -432,28 +453,21 @@ __global__ void __launch_bounds__(k3NT<T>, min_blocks3<T>(8)) batch3d(Inst3<T> *
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Tile3<T> &S = *reinterpret_cast<Tile3<T> *>(smem_raw);
-    // the item at hand, its instance's grid and constants: read again where they are needed. Held
-    // in registers through the march they cost about 30 of its 128, and it spilled: 8 steps of
-    // 15.8 M cells FP64 took 6.6 ms, so 4.7 ms (5.2 ms with the former march).
-    struct Now {
-        int item, inst;
-        Range rg;
-        Grid3 grid;
-        StepConsts<T> c;
-    };
-    __shared__ Now s_now;
+    __shared__ Now<T, Grid3> s_now;
     __shared__ int s_last;
-    const volatile Now &now = s_now;
+    const volatile Now<T, Grid3> &now = s_now;
     const volatile StepConsts<T> &ph = s_now.c;
     const volatile Grid3 &grid = s_now.grid;
     march3d_init(S);
     Ring3 ring;
+    int next = (int)blockIdx.x; // thread 0: the item to take
     for (;;) {
         __syncthreads(); // everyone is done with the previous item
         if (threadIdx.x == 0) {
-            const int w = (int)atomicAdd(counter, 1u);
+            const int w = next;
             s_now.item = w;
             if (w < nitems) {
+                next = (int)(gridDim.x + atomicAdd(counter, 1u)); // (looked at behind this item's march)
                 const int i = items[w].x;
                 const Inst3<T> *I = insts + i;
                 s_now.inst = i;
@@ -573,9 +587,13 @@ __global__ void __launch_bounds__(NT) batch_sums(I *insts, const int2 *items, co
 {
     __shared__ int s_item;
     __shared__ int s_last;
+    int next = (int)blockIdx.x; // thread 0: the item to take
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(counter, 1u);
+        if (threadIdx.x == 0) {
+            s_item = next;
+            if (next < nitems) next = (int)(gridDim.x + atomicAdd(counter, 1u));
+        }
         __syncthreads();
         const int w = s_item;
         if (w >= nitems) break;
@@ -619,7 +637,7 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         else stream_ = stream;
         if (e == cudaSuccess) e = cudaMalloc(&insts_, sizeof(Inst) * cap_);
         if (e == cudaSuccess) e = cudaMalloc(&ranges_, sizeof(Range) * cap_);
-        if (e == cudaSuccess) e = cudaMalloc(&counter_, 64);
+        if (e == cudaSuccess) e = cudaMalloc(&counter_, sizeof(unsigned) * counters_);
         if (e == cudaSuccess) e = cudaMalloc(&scratch_bits_, 64);
         if (e == cudaSuccess) e = cudaMemset(scratch_bits_, 0, 64);
         if (e == cudaSuccess) e = cudaHostAlloc(&status_h_, sizeof(SlotStatus) * cap_, cudaHostAllocMapped);
@@ -672,8 +690,8 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         if (own_stream_) cudaStreamDestroy(stream_);
     }
 
-    // 2D rows are padded to a 16-byte multiple (one spare cell for odd NB_Y in FP32) so
-    // that every instance can be fed by TMA; 3D keeps the reference strides.
+    // 2D rows are padded to a 16-byte multiple (one spare cell for odd NB_Y in FP32); 3D keeps the
+    // reference strides.
     static size_t row_stride(size_t nb_y)
     {
         const size_t per = 16 / (2 * sizeof(T)); // cells per 16 bytes of one pair array
@@ -766,18 +784,9 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         if constexpr (D == 2) {
             I.ys = (long long)ys;
             I.nstrips = (int)((nb_y + kStripW - 1) / kStripW);
-            const size_t rowbytes = 2 * sizeof(T) * ys;
-            const CUtensorMapDataType dt =
-                sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
             for (int b = 0; b < 2; ++b) {
                 I.rhoE[b] = sl.rhoE[b];
                 I.uv[b] = sl.uvx[b];
-                if (!encode_tmap_2d(&I.tm[b][0], dt, sl.rhoE[b], 2 * (nb_y + 2), nb_x + 2, rowbytes, 2 * kStripNT, 1) ||
-                    !encode_tmap_2d(&I.tm[b][1], dt, sl.uvx[b], 2 * (nb_y + 2), nb_x + 2, rowbytes, 2 * kStripNT, 1)) {
-                    free_slot(sl);
-                    set_error(kErrCuda, "batch add: tensor map encoding failed");
-                    return kErrCuda;
-                }
             }
             sl.tiles = I.nstrips;
         } else {
@@ -966,23 +975,23 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         s.tiles = 0;
     }
 
-    void launch()
+    void launch(unsigned *counter)
     {
         if constexpr (D == 2) {
             auto k = fused_ ? batch2d<T, true> : batch2d<T, false>;
-            k<<<blocks_, kStripNT, 0, stream_>>>(insts_, items_, ranges_, nitems_, counter_, parts_, status_d_,
+            k<<<blocks_, kStripNT, 0, stream_>>>(insts_, items_, ranges_, nitems_, counter, parts_, status_d_,
                                                  skip_frac_);
         } else {
             auto k = fused_ ? batch3d<T, true> : batch3d<T, false>;
-            k<<<blocks_, k3NT<T>, smem_, stream_>>>(insts_, items_, ranges_, nitems_, counter_, parts_, status_d_,
+            k<<<blocks_, k3NT<T>, smem_, stream_>>>(insts_, items_, ranges_, nitems_, counter, parts_, status_d_,
                                                    skip_frac_);
         }
     }
 
-    void launch_sums()
+    void launch_sums(unsigned *counter)
     {
         batch_sums<kSumNT, D, T, Inst><<<sum_blocks_, kSumNT, 0, stream_>>>(insts_, sum_list_, ranges_, nsums_,
-                                                                           counter_ + 1, parts_, status_d_);
+                                                                           counter, parts_, status_d_);
     }
 
     // Rows (planes) per step item, at most: the caller's, or the one with the shortest
@@ -1067,20 +1076,26 @@ template <class T, int D> class BatchEngine final : public BatchBase {
             cudaGraphExecDestroy(graph_);
             graph_ = nullptr;
         }
+        if (e == cudaSuccess && (size_t)nsteps + 1 > counters_) {
+            cudaFree(counter_);
+            counter_ = nullptr;
+            counters_ = std::max<size_t>((size_t)nsteps + 1, 2 * counters_);
+            e = cudaMalloc(&counter_, sizeof(unsigned) * counters_);
+            if (e != cudaSuccess) counters_ = 0;
+        }
         if (e == cudaSuccess && nitems_ > 0 && nsteps > 0) {
             cudaGraph_t g = nullptr;
             e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
+            // a counter per step and one for the sums, cleared together (a clear ahead of every
+            // step was a graph node of its own between the kernels)
+            if (e == cudaSuccess) e = cudaMemsetAsync(counter_, 0, sizeof(unsigned) * ((size_t)nsteps + 1), stream_);
             for (int k = 0; k < nsteps && e == cudaSuccess; ++k) {
-                e = cudaMemsetAsync(counter_, 0, sizeof(unsigned), stream_);
-                if (e == cudaSuccess) {
-                    launch();
-                    e = cudaGetLastError();
-                }
+                launch(counter_ + k);
+                e = cudaGetLastError();
             }
             // the conservation sums of the state the run ends on
-            if (e == cudaSuccess) e = cudaMemsetAsync(counter_ + 1, 0, sizeof(unsigned), stream_);
             if (e == cudaSuccess) {
-                launch_sums();
+                launch_sums(counter_ + nsteps);
                 e = cudaGetLastError();
             }
             const cudaError_t e2 = cudaStreamEndCapture(stream_, &g);
@@ -1107,7 +1122,8 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     int2 *items_ = nullptr, *sum_list_ = nullptr;
     size_t items_cap_ = 0;
     ItemPart *parts_ = nullptr;
-    unsigned *counter_ = nullptr;
+    unsigned *counter_ = nullptr; // one per step of the graph and one for the sums
+    size_t counters_ = 256;
     unsigned long long *scratch_bits_ = nullptr;
     SlotStatus *status_h_ = nullptr, *status_d_ = nullptr;
     std::vector<Slot> slots_;

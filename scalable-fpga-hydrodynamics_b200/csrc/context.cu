@@ -241,21 +241,6 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 }
 } // namespace
 
-bool encode_tmap_2d(CUtensorMap *tm, CUtensorMapDataType dt, const void *base, uint64_t dim0, uint64_t dim1,
-                    uint64_t stride1_bytes, uint32_t box0, uint32_t box1)
-{
-    auto fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[2] = {dim0, dim1};
-    cuuint64_t strides[1] = {stride1_bytes};
-    cuuint32_t box[2] = {box0, box1};
-    cuuint32_t es[2] = {1, 1};
-    CUresult r = fn(tm, dt, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
-
 bool encode_tmap_3d(CUtensorMap *tm, CUtensorMapDataType dt, const void *base, uint64_t dim0, uint64_t dim1,
                     uint64_t dim2, uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0, uint32_t box1,
                     uint32_t box2)

@@ -14,17 +14,15 @@
 //
 // Kernels:
 //  strip2d   one CTA = 128 lanes over 128 consecutive columns (126 interior + one
-//            halo column each side), marching down `chunk` rows. Each row arrives in
-//            shared memory through two TMA tile loads (one per array) into a 4-deep
-//            mbarrier ring (or per-lane cp.async where TMA rejects the row pitch); each
-//            lane converts its cell to primitives once, computes the x face below it and
-//            the y face to its right once (neighbour inputs and fluxes exchanged through
-//            shared memory with 128-bit accesses), updates the row behind, stores it with
-//            128-bit stores and folds mass, signal speed and the error checks into the
-//            fused epilogue.
+//            halo column each side), marching down `chunk` rows. Each lane brings its own
+//            cells into a 4-deep shared-memory ring by cp.async, converts each to primitives
+//            once, computes the x face below it and the y face to its right once (neighbour
+//            inputs and fluxes exchanged through shared memory with 128-bit accesses), updates
+//            the row behind, stores it with 128-bit stores and folds mass, signal speed and
+//            the error checks into the fused epilogue.
 //  direct2d  one thread per cell, scalar loads of the 5-point stencil, every face
 //            evaluated from both sides like the reference. Any alignment, any size;
-//            used when the strip kernel's TMA rules do not hold and as a cross-check.
+//            used when a cell is not aligned to its size and as a cross-check.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -109,34 +107,22 @@ template <class T, bool kF = false> __global__ void __launch_bounds__(kRedoNT) r
 }
 
 // ------------------------------------------------------------------- strip kernel ---
-// kTma: rows staged by TMA tile loads (16-byte row pitch), else by per-lane cp.async.
 // kF: fused arithmetic (hydro_math.cuh). kMinB: resident blocks per SM the registers are
 // budgeted for (a launch-shape choice: more blocks, fewer registers per thread).
-template <class T, bool kTma, bool kF, int kMinB = 4>
-__global__ void __launch_bounds__(kStripNT, kMinB)
-    strip2d(const __grid_constant__ CUtensorMap tmr, const __grid_constant__ CUtensorMap tmu, Args2<T> g)
+template <class T, bool kF, int kMinB> __global__ void __launch_bounds__(kStripNT, kMinB) strip2d(Args2<T> g)
 {
     __shared__ Smem2<T> S;
-    if (kTma && threadIdx.x == 0) {
-        prefetch_tensormap(&tmr);
-        prefetch_tensormap(&tmu);
-    }
-    march2d_init(S);
     const int i0 = 1 + g.chunk * (int)blockIdx.y;
-    const March2 geo{kStripW * (int)blockIdx.x, i0, min(i0 + g.chunk - 1, g.nb_x), g.nb_x, g.nb_y, g.ys, g.xwrap,
-                     g.rhoE, g.uv};
+    const March2 geo{kStripW * (int)blockIdx.x, i0, min(i0 + g.chunk - 1, g.nb_x)};
     StepAcc acc;
     const SkipLimits lim = skip_limits(g.scr, g.key);
     const float tlo2 = skip_tlo2(lim.f), ggm1 = g.ggm1;
-    const Phys<T> ph = g.ph;
-    unsigned ld = 0;
-    const bool ok = march2d<T, kTma, kF>(S, &tmr, &tmu, geo, g.rhoE_n, g.uv_n, ph, g.DtDx, g.DtDy, ld,
-                                         [&](const Upd2<T> &o) {
-                                             acc.add_mass(o.r);
-                                             if (!state_below(o, ggm1, tlo2))
-                                                 acc.add_speed(o.r, speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
-                                         });
-    if (!ok) acc.err |= kErrWaitTimeout;
+    const Grid2 grid{g.nb_x, g.nb_y, g.xwrap, g.ys};
+    const StepConsts<T> c(g.ph, g.DtDx, g.DtDy, T(0));
+    march2d<T, kF>(S, g.rhoE, g.uv, g.rhoE_n, g.uv_n, geo, grid, c, [&](const Upd2<T> &o) {
+        acc.add_mass(o.r);
+        if (!state_below(o, ggm1, tlo2)) acc.add_speed(o.r, speed2<T, kF>(o.r, o.u, o.v, o.E, c));
+    });
     step_epilogue<kStripNT, T>(acc, g.scr, g.partials, gridDim.x * gridDim.y, blockIdx.x + blockIdx.y * gridDim.x,
                                g.ph.C_min, g.Dt_next, g.status, g.seq, (double)lim.hist, g.key);
 }
@@ -271,19 +257,21 @@ __global__ void sum_partials_kernel(const double2 *partials, int n, double *out)
 
 // ----------------------------------------------------------------- host drivers ---
 namespace {
-template <class T> CUtensorMapDataType tmap_type();
-template <> CUtensorMapDataType tmap_type<double>() { return CU_TENSOR_MAP_DATA_TYPE_FLOAT64; }
-template <> CUtensorMapDataType tmap_type<float>() { return CU_TENSOR_MAP_DATA_TYPE_FLOAT32; }
-
 bool aligned(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 } // namespace
 
-template <class T> using Strip2 = void (*)(const CUtensorMap, const CUtensorMap, Args2<T>);
+// The register budgets built, in resident blocks per SM: the built-in one (hydro_set_launch_shape
+// names it 4; FP32 7 blocks of 72 registers, 135 GCell/s fused at 8000 x 8000 against 129 with 8),
+// and the other one that it accepts.
+template <class T> constexpr int kBlocks2 = sizeof(T) == 8 ? 4 : 7;
+template <class T> constexpr int kAltBlocks2 = sizeof(T) == 8 ? 5 : 8;
 
-template <class T, int kMinB> Strip2<T> strip2d_form(bool tma, bool fused)
+template <class T> using Strip2 = void (*)(Args2<T>);
+
+template <class T> Strip2<T> strip2d_form(bool alt, bool fused)
 {
-    if (tma) return fused ? strip2d<T, true, true, kMinB> : strip2d<T, true, false, kMinB>;
-    return fused ? strip2d<T, false, true, kMinB> : strip2d<T, false, false, kMinB>;
+    if (alt) return fused ? strip2d<T, true, kAltBlocks2<T>> : strip2d<T, false, kAltBlocks2<T>>;
+    return fused ? strip2d<T, true, kBlocks2<T>> : strip2d<T, false, kBlocks2<T>>;
 }
 
 template <class T>
@@ -329,20 +317,9 @@ int step2d(const T *rhoE, const T *uv, T *rhoE_next, T *uv_next, T *Dt_next, con
     g.xwrap = xwrap ? 1 : 0;
 
     using V2 = typename Vec2<T>::type;
-    const size_t rowbytes = 2 * sizeof(T) * (nb_y + 2);
-    // the strip kernel stages rows by TMA when the arrays are 16-byte aligned and the row
-    // pitch a multiple of 16 bytes, else by per-lane cp.async (cells aligned to their size)
-    bool tma_ok = aligned(rhoE, 16) && aligned(uv, 16) && aligned(rhoE_next, sizeof(V2)) &&
-                  aligned(uv_next, sizeof(V2)) && rowbytes % 16 == 0;
-    CUtensorMap tmr, tmu;
-    std::memset(&tmr, 0, sizeof tmr);
-    std::memset(&tmu, 0, sizeof tmu);
-    if (tma_ok && which != Kernel::Direct) {
-        tma_ok = encode_tmap_2d(&tmr, tmap_type<T>(), rhoE, 2 * (nb_y + 2), nb_x + 2, rowbytes, 2 * kStripNT, 1) &&
-                 encode_tmap_2d(&tmu, tmap_type<T>(), uv, 2 * (nb_y + 2), nb_x + 2, rowbytes, 2 * kStripNT, 1);
-    }
-    const bool strip_ok = tma_ok || (aligned(rhoE, sizeof(V2)) && aligned(uv, sizeof(V2)) &&
-                                     aligned(rhoE_next, sizeof(V2)) && aligned(uv_next, sizeof(V2)));
+    // the strip kernel copies and stores cells whole
+    const bool strip_ok = aligned(rhoE, sizeof(V2)) && aligned(uv, sizeof(V2)) && aligned(rhoE_next, sizeof(V2)) &&
+                          aligned(uv_next, sizeof(V2));
     if (which == Kernel::Strip && !strip_ok) {
         set_error(kErrArg, "step2d: strip kernel needs arrays aligned to their cell size");
         return kErrArg;
@@ -356,9 +333,8 @@ int step2d(const T *rhoE, const T *uv, T *rhoE_next, T *uv_next, T *Dt_next, con
         // rows per block: at most the cap (the tuned value when one is set with
         // hydro_set_launch_shape, else 256), at least 2 (one row per block measured no faster)
         const LaunchShape shape = launch_shape(2, sizeof(T));
-        constexpr int kAltB = sizeof(T) == 8 ? 5 : 8; // the other register budget built
-        const bool alt = shape.blocks == kAltB;
-        const Strip2<T> kern = alt ? strip2d_form<T, kAltB>(tma_ok, fused) : strip2d_form<T, 4>(tma_ok, fused);
+        const bool alt = shape.blocks == kAltBlocks2<T>;
+        const Strip2<T> kern = strip2d_form<T>(alt, fused);
         int per_sm = 1;
         cudaError_t eo = blocks_per_sm(reinterpret_cast<const void *>(kern), kStripNT, 0, &per_sm);
         if (eo != cudaSuccess) {
@@ -377,10 +353,10 @@ int step2d(const T *rhoE, const T *uv, T *rhoE_next, T *uv_next, T *Dt_next, con
         g.partials = ctx->partials;
         ctx->last_warps = 0;
         ctx->last_chunk = chunk;
-        ctx->last_tma = tma_ok;
+        ctx->last_tma = false;
         const dim3 grid(nstrips, nchunks);
-        ctx->last_blocks = alt ? kAltB : 4;
-        kern<<<grid, kStripNT, 0, stream>>>(tmr, tmu, g);
+        ctx->last_blocks = alt ? kAltBlocks2<T> : 4;
+        kern<<<grid, kStripNT, 0, stream>>>(g);
     } else {
         const int gx = (int)((nb_y + kDirectNT - 1) / kDirectNT);
         const int gy = (int)std::min<size_t>(nb_x, 65535);
@@ -716,13 +692,7 @@ extern "C" int hydro2d_step_f64_noalloc(const double *d_rhoE, const double *d_uv
     g.ggm1 = skip_ggm1(gamma, gamma_minus_one);
     g.xwrap = 1;
 
-    const size_t rowbytes = 2 * sizeof(T) * (NB_Y + 2);
-    bool strip_ok = aligned(d_rhoE, 16) && aligned(d_uv, 16) && aligned(d_rhoE_next, 16) && aligned(d_uv_next, 16) &&
-                    rowbytes % 16 == 0;
-    CUtensorMap tmr, tmu;
-    if (strip_ok)
-        strip_ok = encode_tmap_2d(&tmr, tmap_type<T>(), d_rhoE, 2 * (NB_Y + 2), NB_X + 2, rowbytes, 2 * kStripNT, 1) &&
-                   encode_tmap_2d(&tmu, tmap_type<T>(), d_uv, 2 * (NB_Y + 2), NB_X + 2, rowbytes, 2 * kStripNT, 1);
+    const bool strip_ok = aligned(d_rhoE, 16) && aligned(d_uv, 16) && aligned(d_rhoE_next, 16) && aligned(d_uv_next, 16);
     int chunk = 0;
     unsigned gx = 0, gy = 0;
     if (!noalloc_shape(NB_X, NB_Y, strip_ok, device_sms(), &chunk, &gx, &gy)) {
@@ -732,7 +702,7 @@ extern "C" int hydro2d_step_f64_noalloc(const double *d_rhoE, const double *d_uv
     g.chunk = chunk;
     const int kernel = (int)(strip_ok ? Kernel::Strip : Kernel::Direct);
     if (strip_ok)
-        strip2d<T, true, false><<<dim3(gx, gy), kStripNT, 0, st>>>(tmr, tmu, g);
+        strip2d<T, false, kBlocks2<T>><<<dim3(gx, gy), kStripNT, 0, st>>>(g);
     else
         direct2d<T><<<dim3(gx, gy), kDirectNT, 0, st>>>(g);
     // the redo pass returns at once unless the step left Dt_next to it

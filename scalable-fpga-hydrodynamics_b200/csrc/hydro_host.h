@@ -77,7 +77,7 @@ inline unsigned long long problem_key(const void *dt_next, size_t a, size_t b, s
 struct LaunchShape {
     int warps = 0;  // 3D: warps per block (tile rows with halo)
     int chunk = 0;  // rows (2D) or planes (3D) each block marches
-    int blocks = 0; // 2D: resident blocks per SM the registers are budgeted for (4, or 5 in FP64 / 8 in FP32)
+    int blocks = 0; // 2D: register budget, 4 (the built-in one) or 5 in FP64 / 8 in FP32 blocks per SM
 };
 LaunchShape launch_shape(int dim, size_t tsize);
 int set_launch_shape(int dim, size_t tsize, int warps, int chunk, int blocks);
@@ -114,10 +114,8 @@ enum : int {
     kErrTimeout = -4,
 };
 
-// Encode a 2D tiled tensor map (no swizzle, zero OOB fill). Returns false when the
+// Encode a 3D tiled tensor map (no swizzle, zero OOB fill). Returns false when the
 // driver entry point is missing or encoding fails.
-bool encode_tmap_2d(CUtensorMap *tm, CUtensorMapDataType dt, const void *base, uint64_t dim0, uint64_t dim1,
-                    uint64_t stride1_bytes, uint32_t box0, uint32_t box1);
 bool encode_tmap_3d(CUtensorMap *tm, CUtensorMapDataType dt, const void *base, uint64_t dim0, uint64_t dim1,
                     uint64_t dim2, uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t box0, uint32_t box1,
                     uint32_t box2);

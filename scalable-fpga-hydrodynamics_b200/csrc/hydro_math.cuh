@@ -205,6 +205,13 @@ template <class T> struct Vec2;
 template <> struct Vec2<double> { using type = double2; };
 template <> struct Vec2<float> { using type = float2; };
 
+// x with the bits of `mask` (0 or the sign bit) of its high word flipped
+__device__ __forceinline__ double flip_sign(double x, unsigned mask)
+{
+    return __hiloint2double((int)((unsigned)__double2hiint(x) ^ mask), __double2loint(x));
+}
+__device__ __forceinline__ float flip_sign(float x, unsigned mask) { return __uint_as_float(__float_as_uint(x) ^ mask); }
+
 // std::max(a, b) as the reference calls it: a unless a < b
 template <class T> __device__ __forceinline__ T smax(T a, T b) { return (a < b) ? b : a; }
 

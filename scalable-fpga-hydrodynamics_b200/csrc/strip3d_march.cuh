@@ -49,13 +49,6 @@ constexpr int k3TZ = 30; // interior columns per tile
 
 __device__ __forceinline__ int wrap_plane(int n, int nb_x) { return n == 0 ? nb_x : (n == nb_x + 1 ? 1 : n); }
 
-// x with the bits of `mask` (0 or the sign bit) of its high word flipped
-__device__ __forceinline__ double flip_sign(double x, unsigned mask)
-{
-    return __hiloint2double((int)((unsigned)__double2hiint(x) ^ mask), __double2loint(x));
-}
-__device__ __forceinline__ float flip_sign(float x, unsigned mask) { return __uint_as_float(__float_as_uint(x) ^ mask); }
-
 template <class T> __device__ __forceinline__ typename Vec2<T>::type pair3(T a, T b)
 {
     typename Vec2<T>::type v;
