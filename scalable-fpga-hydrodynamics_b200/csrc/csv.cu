@@ -14,9 +14,17 @@
 // move N to the correctly rounded value.
 //
 // Pipeline, per chunk of rows: one thread formats one cell's line into a fixed-size slot,
-// a device scan of the line lengths gives each line's offset, a compaction writes the
-// lines back to back, and the chunk goes to pinned host memory while the next chunk is
-// formatted; the host writes the bytes to the file.
+// a device scan of the line lengths gives each line's offset, and a compaction writes the
+// lines back to back; while the next chunk is formatted, this one goes to the host in pieces
+// through two pinned buffers, each copied while the host writes the other to the file.
+//
+// The kernels of a 1200 x 800 FP64 file (28.6 MB) take 0.6 ms together; what bounds the call is
+// the host: the write itself (about 8 ms into the page cache) and the allocations. Pinned memory
+// is the expensive one (1.5 to 4 ms per MB to allocate and free), so only two pieces of 384 KB are
+// pinned. That file took 121 to 220 ms with whole chunks pinned (4 M cells, 112 bytes a line);
+// with these pieces it takes 10 to 20, of which 2 are left when written to /dev/null (pieces of
+// 1 MB: 5.5; 2 MB: 8.5). A chunk of 64 K cells keeps the device's share at 22 MB and its kernels
+// behind the writing of the chunk before; 16 K cells leave 4 ms, 256 K no less than 2.
 #include <cub/device/device_scan.cuh>
 
 #include <math.h>
@@ -335,98 +343,117 @@ long long write_csv(const T *rhoE, const T *uvx, size_t nb_x, size_t nb_y, size_
         return total;
     }
     // cells per chunk (HYDRO_B200_CSV_CHUNK_CELLS overrides, e.g. to exercise many chunks)
-    long long target = 4ll << 20;
+    long long target = 1ll << 16;
     if (const char *env = getenv("HYDRO_B200_CSV_CHUNK_CELLS")) {
         const long long v = atoll(env);
         if (v > 0) target = v;
     }
     const int rows = (int)std::max<long long>(1, std::min<long long>((long long)nb_x, target / per_row));
     const long long cap = per_row * rows;
-    char *slots = nullptr, *out = nullptr, *host[2] = {nullptr, nullptr};
-    unsigned *lens = nullptr;
-    unsigned long long *offs = nullptr, *h_tot = nullptr;
-    void *tmp = nullptr;
+    const size_t line_bytes = (size_t)cap * kSlot;
+    const size_t piece = std::min<size_t>(line_bytes, (size_t)384 << 10);
+    // device: the slots, two buffers of lines back to back, lengths, offsets, the scan's scratch
     size_t tmp_bytes = 0;
-    cudaEvent_t done[2] = {nullptr, nullptr};
-    long long pending[2] = {0, 0};
-    cudaError_t e = cudaMalloc(&slots, (size_t)cap * kSlot);
-    if (e == cudaSuccess) e = cudaMalloc(&out, (size_t)cap * kSlot);
-    if (e == cudaSuccess) e = cudaMalloc(&lens, (size_t)cap * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMalloc(&offs, (size_t)(cap + 1) * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMallocHost(&host[0], (size_t)cap * kSlot);
-    if (e == cudaSuccess) e = cudaMallocHost(&host[1], (size_t)cap * kSlot);
-    if (e == cudaSuccess) e = cudaMallocHost(&h_tot, 2 * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done[0], cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done[1], cudaEventDisableTiming);
+    cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (unsigned *)nullptr, (unsigned long long *)nullptr,
+                                                  (int)cap, st);
+    const auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+    const bool many = rows < (int)nb_x; // more than one chunk
+    char *dev = nullptr, *out[2] = {nullptr, nullptr}, *host[2] = {nullptr, nullptr};
+    unsigned long long *h_tot = nullptr; // per chunk parity: the last line's offset and length
+    cudaEvent_t ready[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
+    cudaStream_t copies = nullptr;
     if (e == cudaSuccess)
-        e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, lens, offs, (int)cap, st);
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, tmp_bytes);
+        e = cudaMalloc(&dev, up(line_bytes) * (many ? 3 : 2) + up(cap * sizeof(unsigned)) +
+                                 up(cap * sizeof(unsigned long long)) + tmp_bytes);
+    char *const slots = dev;
+    unsigned *lens = nullptr;
+    unsigned long long *offs = nullptr;
+    void *tmp = nullptr;
+    if (e == cudaSuccess) {
+        char *q = dev + up(line_bytes);
+        out[0] = q;
+        if (many) q += up(line_bytes);
+        out[1] = q;
+        q += up(line_bytes);
+        lens = reinterpret_cast<unsigned *>(q);
+        q += up(cap * sizeof(unsigned));
+        offs = reinterpret_cast<unsigned long long *>(q);
+        tmp = q + up(cap * sizeof(unsigned long long));
+        char *pinned = nullptr;
+        e = cudaMallocHost(&pinned, 2 * up(piece) + 4 * sizeof(unsigned long long));
+        if (e == cudaSuccess) {
+            host[0] = pinned;
+            host[1] = pinned + up(piece);
+            h_tot = reinterpret_cast<unsigned long long *>(pinned + 2 * up(piece));
+        }
+    }
+    for (int b = 0; b < 2; ++b) {
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ready[b], cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&copied[b], cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&copies, cudaStreamNonBlocking);
+
+    // the lines of chunk c, whose kernels have been launched, to the file
+    auto write_chunk = [&](int c) {
+        const int b = c & 1;
+        e = cudaEventSynchronize(ready[b]);
+        if (e != cudaSuccess) return;
+        const size_t bytes = (size_t)h_tot[2 * b] + (unsigned)h_tot[2 * b + 1];
+        auto fetch = [&](size_t at, int h) {
+            e = cudaMemcpyAsync(host[h], out[b] + at, std::min(piece, bytes - at), cudaMemcpyDeviceToHost, copies);
+            if (e == cudaSuccess) e = cudaEventRecord(copied[h], copies);
+        };
+        int h = 0;
+        fetch(0, h);
+        for (size_t at = 0; e == cudaSuccess && at < bytes; at += piece, h ^= 1) {
+            if (at + piece < bytes) fetch(at + piece, h ^ 1); // while this piece is written
+            if (e == cudaSuccess) e = cudaEventSynchronize(copied[h]);
+            if (e != cudaSuccess) return;
+            const size_t n = std::min(piece, bytes - at);
+            if (fwrite(host[h], 1, n, f) != n) {
+                set_error(kErrArg, "write_csv: short write to %s", path);
+                rc = kErrArg;
+                return;
+            }
+            total += (long long)n;
+        }
+    };
     int chunk = 0;
-    for (long long row0 = 1; e == cudaSuccess && row0 <= (long long)nb_x; row0 += rows, ++chunk) {
+    for (long long row0 = 1; e == cudaSuccess && rc == kOk && row0 <= (long long)nb_x; row0 += rows, ++chunk) {
         const int nr = (int)std::min<long long>(rows, (long long)nb_x - row0 + 1);
         const long long n = per_row * nr;
+        const int b = chunk & 1;
         const int blocks = (int)std::min<long long>((n + 255) / 256, (long long)device_sms() * 16);
         format_lines<T, D><<<blocks, 256, 0, st>>>(rhoE, uvx, (int)nb_y, (int)nb_z, row0, nr, (long long)i_offset,
                                                     slots, lens);
         e = cudaGetLastError();
-        // offsets of the n lines; offs[n] = the chunk's byte count
+        // offsets of the n lines
         if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, lens, offs, (int)n, st);
+        if (e == cudaSuccess) {
+            compact_lines<<<blocks, 256, 0, st>>>(slots, lens, offs, n, out[b]);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) h_tot[2 * b + 1] = 0; // (a 4-byte length in an 8-byte word)
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&h_tot[0], offs + (n - 1), sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-        unsigned last_len = 0;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h_tot[1], lens + (n - 1), sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) break;
-        memcpy(&last_len, &h_tot[1], sizeof(unsigned));
-        const long long bytes = (long long)h_tot[0] + last_len;
-        compact_lines<<<blocks, 256, 0, st>>>(slots, lens, offs, n, out);
-        e = cudaGetLastError();
-        const int b = chunk & 1;
-        // the previous use of this pinned buffer has been written out below
-        if (e == cudaSuccess) e = cudaMemcpyAsync(host[b], out, (size_t)bytes, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaEventRecord(done[b], st);
-        pending[b] = bytes;
-        // write the other buffer (the previous chunk) while this one is in flight
-        const int o = b ^ 1;
-        if (e == cudaSuccess && pending[o] > 0 && chunk > 0) {
-            e = cudaEventSynchronize(done[o]);
-            if (e == cudaSuccess) {
-                if ((long long)fwrite(host[o], 1, (size_t)pending[o], f) != pending[o]) {
-                    set_error(kErrArg, "write_csv: short write to %s", path);
-                    rc = kErrArg;
-                    break;
-                }
-                total += pending[o];
-                pending[o] = 0;
-            }
-        }
+            e = cudaMemcpyAsync(&h_tot[2 * b], offs + (n - 1), sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&h_tot[2 * b + 1], lens + (n - 1), sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaEventRecord(ready[b], st);
+        // the previous chunk, whose buffer the next one takes over
+        if (e == cudaSuccess && chunk > 0) write_chunk(chunk - 1);
     }
-    // the last chunk
-    if (e == cudaSuccess && rc == kOk) {
-        const int b = (chunk - 1) & 1;
-        if (pending[b] > 0) {
-            e = cudaEventSynchronize(done[b]);
-            if (e == cudaSuccess) {
-                if ((long long)fwrite(host[b], 1, (size_t)pending[b], f) != pending[b]) {
-                    set_error(kErrArg, "write_csv: short write to %s", path);
-                    rc = kErrArg;
-                } else {
-                    total += pending[b];
-                }
-            }
-        }
+    if (e == cudaSuccess && rc == kOk && chunk > 0) write_chunk(chunk - 1);
+    cudaStreamSynchronize(st); // (after an error work may still be in flight)
+    if (copies) {
+        cudaStreamSynchronize(copies);
+        cudaStreamDestroy(copies);
     }
-    if (e != cudaSuccess) cudaStreamSynchronize(st);
-    cudaFree(slots);
-    cudaFree(out);
-    cudaFree(lens);
-    cudaFree(offs);
-    cudaFree(tmp);
+    cudaFree(dev);
     if (host[0]) cudaFreeHost(host[0]);
-    if (host[1]) cudaFreeHost(host[1]);
-    if (h_tot) cudaFreeHost(h_tot);
-    for (auto ev : done)
-        if (ev) cudaEventDestroy(ev);
+    for (int b = 0; b < 2; ++b) {
+        if (ready[b]) cudaEventDestroy(ready[b]);
+        if (copied[b]) cudaEventDestroy(copied[b]);
+    }
     if (fclose(f) != 0 && rc == kOk) {
         set_error(kErrArg, "write_csv: closing %s failed", path);
         rc = kErrArg;

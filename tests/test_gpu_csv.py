@@ -99,3 +99,26 @@ def test_write_csv_many_chunks(cuda, chunk_cells, tmp_path, monkeypatch):
     out = tmp_path / "gpu.csv"
     hb.write_csv(run.cur, nb, out)
     assert out.read_bytes() == files[0].read_bytes()
+
+
+@pytest.mark.parametrize("T", [np.float64, np.float32])
+@pytest.mark.parametrize("nb,chunk", [((1, 1), None), ((300, 251), None), ((61, 250), 1 << 20), ((13, 3001), 4000),
+                                      ((40, 30, 20), 7), ((40, 31, 21), None)])
+def test_write_csv_pieces_and_chunks(cuda, nb, chunk, T, tmp_path, monkeypatch):
+    """Lines built on the host: a file below one piece, chunks of several pieces with a ragged
+    last one (the default chunk and all cells at once), many chunks, a last chunk of one row."""
+    import torch
+    D, rng = len(nb), np.random.default_rng(3)
+    shape = tuple(n + 2 for n in nb)
+    q, v = (rng.uniform(-30, 30, shape + (n,)).astype(T) for n in (2, D))
+    if chunk:
+        monkeypatch.setenv("HYDRO_B200_CSV_CHUNK_CELLS", str(chunk))
+    out = tmp_path / "gpu.csv"
+    n = hb.write_csv([torch.from_numpy(a).cuda() for a in (q, v)], nb, out, i_offset=2)
+    inner = tuple(slice(1, -1) for _ in nb)
+    cells = np.concatenate([q[inner], v[inner]], axis=-1).reshape(-1, 2 + D).astype(np.float64)
+    head = "x,y,rho,p,u,v" if D == 2 else "x,y,z,rho,p,u,v,w"
+    lines = [",".join([str(i + 2 * (a == 0)) for a, i in enumerate(idx)] + ["%g" % x for x in row])
+             for idx, row in zip(np.ndindex(nb), cells.tolist())]
+    want = "\n".join([head] + lines + [""]).encode()
+    assert n == len(want) and out.read_bytes() == want
