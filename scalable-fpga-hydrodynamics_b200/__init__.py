@@ -415,9 +415,11 @@ class BlastRun:
         (self.stream or torch.cuda.current_stream()).synchronize()
         info = StepInfo()
         _check(lib().hydro_last_step_info(ctypes.byref(info)))
+        self._advance(info, self.T(self.dt_dev.item()))
+
+    def _advance(self, info, dtn):
         self.last_info = info
         self.cur, self.nxt = self.nxt, self.cur
-        dtn = self.T(self.dt_dev.item())
         big = self.T(1e20)
         self.dt = dtn if dtn < big else big
         self.t_log.append(self.t)
@@ -426,8 +428,16 @@ class BlastRun:
         self.t += float(self.dt)
 
     def step(self):
-        self.step_kernel_only()
-        self.step_finish()
+        """One launch and one wait. Waiting in the step itself, the library launches the
+        signal-speed pass over all cells only when it is needed (step_kernel_only, which does not
+        wait, has to enqueue it each time), and the new Dt is C_min / max_speed of the step's
+        record, the division that the kernel writes to dt_dev, in place of a copy back: 1024 x 1024
+        FP64 63 us per step with the two, 49 without."""
+        _, info = step(self.cur, self.nxt, self.dt_dev, self.phys, self.phys.dtd(self.dt), kernel=self.kernel,
+                       stream=self.stream, arith=self.arith)
+        with np.errstate(all="ignore"):
+            dtn = self.T(self.phys.C_min) / self.T(info.max_speed)
+        self._advance(info, dtn)
 
     def run(self, max_t: float, max_it: int):
         while self.t < max_t and self.it < max_it:
