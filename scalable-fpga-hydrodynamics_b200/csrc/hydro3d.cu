@@ -37,7 +37,7 @@ template <class T> struct Args3 {
     Grid3 grid;
     int nb_x, nb_y, nb_z;
     long long zs, zy;
-    int chunk;
+    Chunks chunks; // of the strip kernel's planes
     StepScratch *scr;
     double2 *partials;
     StepStatus *status;
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(32 * SM::W, min_blocks3<T>(SM::W))
         prefetch_tensormap(&tmu);
     }
     march3d_init(S);
-    const int i0 = 1 + g.chunk * (int)blockIdx.z;
-    const March3 geo{k3TZ * (int)blockIdx.x, (SM::R - 2) * (int)blockIdx.y, i0, min(i0 + g.chunk - 1, g.nb_x)};
+    const int i0 = g.chunks.begin((int)blockIdx.z), i1 = g.chunks.begin((int)blockIdx.z + 1) - 1;
+    const March3 geo{k3TZ * (int)blockIdx.x, (SM::R - 2) * (int)blockIdx.y, i0, min(i1, g.nb_x)};
     StepAcc acc;
     const SkipLimits lim = skip_limits(g.scr, g.key);
     const float tlo2 = skip_tlo2(lim.f), ggm1 = g.ggm1;
@@ -323,13 +323,8 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
             set_error(kErrCuda, "step3d: %s", cudaGetErrorString(ea));
             return kErrCuda;
         }
-        int chunk = march_chunk(nb_x, (size_t)nz * ny, per_sm, shape.chunk > 0 ? shape.chunk : 256, 3);
-        int nchunks = (int)((nb_x + chunk - 1) / chunk);
-        if (nchunks > 65535) {
-            chunk = (int)((nb_x + 65534) / 65535);
-            nchunks = (int)((nb_x + chunk - 1) / chunk);
-        }
-        g.chunk = chunk;
+        g.chunks = march_chunks(nb_x, (size_t)nz * ny, per_sm, shape.chunk, 3);
+        const int nchunks = g.chunks.count;
         nblocks = (unsigned)nz * ny * nchunks;
         if ((err = ctx_reserve(ctx, nblocks)) != kOk) return err;
         g.partials = ctx->partials;
@@ -355,7 +350,7 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
             return kErrCuda;
         }
         ctx->last_warps = rows;
-        ctx->last_chunk = chunk;
+        ctx->last_chunk = g.chunks.longs > 0 ? g.chunks.len : g.chunks.rest;
         ctx->last_blocks = min_blocks3<T>(W);
         ctx->last_tma = tma;
     } else {
@@ -367,7 +362,7 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
         nblocks = (unsigned)gx * gy * gz;
         if ((err = ctx_reserve(ctx, nblocks)) != kOk) return err;
         g.partials = ctx->partials;
-        g.chunk = 0;
+        g.chunks = Chunks{};
         direct3d<T><<<dim3(gx, gy, gz), dim3(32, 4), 0, stream>>>(g);
     }
     cudaError_t e = cudaGetLastError();

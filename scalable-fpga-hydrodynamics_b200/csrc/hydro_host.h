@@ -94,8 +94,16 @@ int device_sms();
 cudaError_t blocks_per_sm(const void *kernel, int threads, int smem, int *blocks);
 // Rows (2D) or planes (3D) that each block of a march takes: `rows` of them over `tiles`
 // columns of blocks, `per_sm` resident blocks per SM, at most `cap` and at least `least` rows
-// per block (context.cu).
-int march_chunk(size_t rows, size_t tiles, int per_sm, int cap, int least);
+// per block (context.cu). *cost: the launch's time by its model, in rows of one full SM.
+int march_chunk(size_t rows, size_t tiles, int per_sm, int cap, int least, double *cost = nullptr);
+// How the planes of a column of tiles are split in two lengths: `longs` chunks of `len` planes,
+// then chunks of `rest` to the end, `count` in all (Chunks::begin: a chunk's first plane).
+struct Chunks {
+    int longs, len, rest, count;
+    __host__ __device__ int begin(int k) const { return 1 + (k < longs ? k * len : longs * len + (k - longs) * rest); }
+};
+// The split by march_chunk's model; all chunks alike (longs 0) when `cap` > 0 was asked for.
+Chunks march_chunks(size_t rows, size_t tiles, int per_sm, int cap, int least);
 // Grow the partials array to at least n entries (synchronises the device on growth).
 int ctx_reserve(DevCtx *c, size_t n);
 

@@ -67,3 +67,12 @@ def test_chunks(cuda, oracle, T, chunk):
         assert hb.last_launch_shape()["chunk"] <= chunk
     finally:
         hb.set_launch_shape(3, T, 0, 0, 0)
+
+
+@pytest.mark.parametrize("T", [np.float64, np.float32])
+@pytest.mark.parametrize("nb, chunk", [((150, 150, 150), 48), ((151, 151, 149), None), ((3001, 13, 59), None)])
+def test_long_and_short_chunks(cuda, oracle, nb, T, chunk):
+    """Columns split in two lengths of chunk, with a ragged last one."""
+    _run(cuda, oracle, nb, T, 0, False)
+    if chunk and T is np.float64:
+        assert hb.last_launch_shape()["chunk"] == chunk
