@@ -391,7 +391,10 @@ long long write_csv(const T *rhoE, const T *uvx, size_t nb_x, size_t nb_y, size_
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ready[b], cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&copied[b], cudaEventDisableTiming);
     }
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&copies, cudaStreamNonBlocking);
+    // (one chunk is copied behind its kernels: creating the stream took a quarter of the 0.3 ms of a
+    // 60 x 60 file)
+    if (e == cudaSuccess && many) e = cudaStreamCreateWithFlags(&copies, cudaStreamNonBlocking);
+    const cudaStream_t from = many ? copies : st;
 
     // the lines of chunk c, whose kernels have been launched, to the file
     auto write_chunk = [&](int c) {
@@ -400,8 +403,8 @@ long long write_csv(const T *rhoE, const T *uvx, size_t nb_x, size_t nb_y, size_
         if (e != cudaSuccess) return;
         const size_t bytes = (size_t)h_tot[2 * b] + (unsigned)h_tot[2 * b + 1];
         auto fetch = [&](size_t at, int h) {
-            e = cudaMemcpyAsync(host[h], out[b] + at, std::min(piece, bytes - at), cudaMemcpyDeviceToHost, copies);
-            if (e == cudaSuccess) e = cudaEventRecord(copied[h], copies);
+            e = cudaMemcpyAsync(host[h], out[b] + at, std::min(piece, bytes - at), cudaMemcpyDeviceToHost, from);
+            if (e == cudaSuccess) e = cudaEventRecord(copied[h], from);
         };
         int h = 0;
         fetch(0, h);
