@@ -7,18 +7,19 @@
 // (strip2d_march.cuh / strip3d_march.cuh), so an instance's state after n batched steps
 // is bit-identical to n plain steps in the same precision. 2D instances keep the pair
 // layout with rows padded to 16 bytes; 3D instances keep the reference's
-// pair/triple layout (row copies). Work is a flat list of (instance, tile x chunk)
-// items; persistent blocks take one item each by their number and more from an atomic counter.
-// Every item writes its max signal speed and error bits to its own slot; the item that completes an instance's
-// step (ticket per instance) merges that instance's slots -- the result depends neither
-// on which block ran which item nor on the other instances in the batch -- and advances
+// pair/triple layout (row copies). Work is a flat list of items, rows or planes of a strip or
+// tile of an instance, long ones first and short ones last; persistent blocks take one item each by
+// their number and more from an atomic counter. Every item writes its max signal speed and error
+// bits to its own slot; the item that completes an instance's step (ticket per instance) merges
+// that instance's slots -- the result depends neither on which block ran which item nor on how
+// the rows were cut nor on the other instances in the batch -- and advances
 // the instance on the device:
 //   Dt = min(1e20, C_min / max_speed)   (hydro2d/kernel.cxx:318, main.cxx:706-781)
 //   t += Dt (FP64 accumulator), DtDx = Dt / DX ... (main.cxx:703-704, in T)
 //   active while t < t_end and steps < max_steps (main.cxx:689)
 // so a step needs no host round trip and n steps are captured as one CUDA graph. The
 // graph ends with one pass over the final state that forms each instance's compensated
-// FP64 conservation sums (mass, momenta, energy) over the same items, merged per
+// FP64 conservation sums (mass, momenta, energy) over items of its own, merged per
 // instance in a fixed order (the step kernels carry no sums: fewer registers, more
 // resident blocks). The signal speed uses the plain path's exact skip (see
 // batch_threshold).
@@ -68,10 +69,15 @@ template <class T> struct alignas(128) Inst3 {
     unsigned done_items, err;
 };
 
-// An instance's share of the work lists: its step items (parts slots first .. first+count-1, each
-// `chunk` rows or planes of a strip or tile) and its items of the end-of-run sums.
+// A step item: rows (planes) i0 to i1 of one strip (tx) or tile (tx along Z, ty along Y) of an
+// instance; its slot of the parts, and the slots of all of the instance's items.
+struct __align__(16) Item {
+    int inst, part, tx, ty, i0, i1, first, count;
+};
+
+// An instance's share of the items of the end-of-run sums.
 struct Range {
-    int first, count, chunk, sum_first, sum_count;
+    int sum_first, sum_count;
 };
 
 struct ItemPart {
@@ -377,20 +383,28 @@ __device__ __forceinline__ bool publish_item(BatchAcc &acc, ItemPart *parts, int
 // are needed. Held in registers through the march they cost about 30 of its 128 in 3D FP64, and
 // it spilled: 8 steps of 15.8 M cells took 6.6 ms, so 4.7 ms (5.2 ms with the former march).
 template <class T, class Grid> struct Now {
-    int item, inst;
-    Range rg;
+    int w;   // index of the item
+    Item it;
     Grid grid;
     StepConsts<T> c;
 };
+
+// Thread 0: the block's next item. Taken when the one before is done: taken ahead, at its start, a
+// block with a long item held back the one after it (10 steps of 24 2D instances 1145 against
+// 1070 us).
+__device__ __forceinline__ void next_item(int &next, unsigned *counter)
+{
+    if (threadIdx.x == 0) next = (int)(gridDim.x + atomicAdd(counter, 1u));
+}
 
 // resident blocks per SM the register budget of the 2D step aims at
 template <class T> struct Batch2dOcc { static constexpr int value = sizeof(T) == 4 ? 6 : 4; };
 
 // kF: fused arithmetic (hydro_math.cuh)
 template <class T, bool kF>
-__global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<T> *insts, const int2 *items, const Range *ranges,
-                                                      int nitems, unsigned *counter, ItemPart *parts,
-                                                      SlotStatus *status, double skip_frac)
+__global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<T> *insts, const Item *items, int nitems,
+                                                                             unsigned *counter, ItemPart *parts,
+                                                                             SlotStatus *status, double skip_frac)
 {
     __shared__ Smem2<T> S;
     __shared__ Now<T, Grid2> s_now;
@@ -401,43 +415,43 @@ __global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<
         __syncthreads(); // everyone is done with the previous item
         if (threadIdx.x == 0) {
             const int w = next;
-            s_now.item = w;
+            s_now.w = w;
             if (w < nitems) {
-                next = (int)(gridDim.x + atomicAdd(counter, 1u)); // (looked at behind this item's march)
-                const int i = items[w].x;
-                const Inst2<T> *I = insts + i;
-                s_now.inst = i;
-                s_now.rg = ranges[i];
+                const Item it = items[w];
+                const Inst2<T> *I = insts + it.inst;
+                s_now.it = it;
                 s_now.grid = Grid2{I->nb_x, I->nb_y, 1, I->ys};
                 s_now.c = StepConsts<T>(I->ph, I->DtDx, I->DtDy, T(0), (T)I->ggm1,
                                         (T)skip_tlo2(batch_threshold(I, skip_frac)));
             }
         }
         __syncthreads();
-        if (now.item >= nitems) break;
+        if (now.w >= nitems) break;
         MaxAcc acc;
         {
-            const Inst2<T> *I = insts + now.inst;
-            if (!I->active) continue;
-            const int par = I->parity, y = items[now.item].y;
-            const int strip = y % I->nstrips, ck = y / I->nstrips;
-            const int i0 = 1 + ck * now.rg.chunk;
+            const Inst2<T> *I = insts + now.it.inst;
+            if (!I->active) {
+                next_item(next, counter);
+                continue;
+            }
+            const int par = I->parity;
             // (the constants stay in shared memory, the grid is copied: 24 instances of 10.4 M cells,
             // 10 steps FP32 1183 us fused and 1184 strict, FP64 1734 strict; all in shared memory
             // 1228 fused, constants copied 1230 FP32 strict and 1739 FP64)
             const volatile StepConsts<T> &ph = s_now.c;
             const Grid2 grid = s_now.grid;
-            const March2 geo{kStripW * strip, i0, min(i0 + now.rg.chunk - 1, I->nb_x)};
+            const March2 geo{kStripW * now.it.tx, now.it.i0, now.it.i1};
             march2d<T, kF>(S, I->rhoE[par], I->uv[par], I->rhoE[par ^ 1], I->uv[par ^ 1], geo, grid, ph,
                            [&](const Upd2<T> &o) {
                                if (!state_below(o, ph.ggm1, ph.tlo2))
                                    acc.add_speed(o.r, (double)speed2<T, kF>(o.r, o.u, o.v, o.E, ph));
                            });
         }
-        Inst2<T> *I = insts + now.inst;
-        const int first = now.rg.first, count = now.rg.count;
-        if (publish_step<kStripNT>(acc, parts, now.item, &I->done_items, count, &s_last))
-            finalize_step<kStripNT, T, kF>(I, parts + first, count, status ? status + now.inst : nullptr, skip_frac);
+        next_item(next, counter); // (in flight while the item's result is published)
+        Inst2<T> *I = insts + now.it.inst;
+        const int first = now.it.first, count = now.it.count;
+        if (publish_step<kStripNT>(acc, parts, now.it.part, &I->done_items, count, &s_last))
+            finalize_step<kStripNT, T, kF>(I, parts + first, count, status ? status + now.it.inst : nullptr, skip_frac);
     }
 }
 
@@ -447,9 +461,9 @@ template <class T> constexpr int k3NT = 32 * Tile3<T>::W;
 template <class T> constexpr int k3TY = Tile3<T>::R - 2; // interior rows per tile
 
 template <class T, bool kF>
-__global__ void __launch_bounds__(k3NT<T>, min_blocks3<T>(8)) batch3d(Inst3<T> *insts, const int2 *items,
-                                                                      const Range *ranges, int nitems, unsigned *counter,
-                                                                      ItemPart *parts, SlotStatus *status, double skip_frac)
+__global__ void __launch_bounds__(k3NT<T>, min_blocks3<T>(8)) batch3d(Inst3<T> *insts, const Item *items, int nitems,
+                                                                      unsigned *counter, ItemPart *parts,
+                                                                      SlotStatus *status, double skip_frac)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Tile3<T> &S = *reinterpret_cast<Tile3<T> *>(smem_raw);
@@ -465,29 +479,27 @@ __global__ void __launch_bounds__(k3NT<T>, min_blocks3<T>(8)) batch3d(Inst3<T> *
         __syncthreads(); // everyone is done with the previous item
         if (threadIdx.x == 0) {
             const int w = next;
-            s_now.item = w;
+            s_now.w = w;
             if (w < nitems) {
-                next = (int)(gridDim.x + atomicAdd(counter, 1u)); // (looked at behind this item's march)
-                const int i = items[w].x;
-                const Inst3<T> *I = insts + i;
-                s_now.inst = i;
-                s_now.rg = ranges[i];
+                const Item it = items[w];
+                const Inst3<T> *I = insts + it.inst;
+                s_now.it = it;
                 s_now.grid = Grid3(I->nb_x, I->nb_y, I->nb_z, 1);
                 s_now.c = StepConsts<T>(I->ph, I->DtDx, I->DtDy, I->DtDz, (T)I->ggm1,
                                         (T)skip_tlo2(batch_threshold(I, skip_frac)));
             }
         }
         __syncthreads();
-        if (now.item >= nitems) break;
+        if (now.w >= nitems) break;
         MaxAcc acc;
         {
-            const Inst3<T> *I = insts + now.inst;
-            if (!I->active) continue;
-            const int par = I->parity, y = items[now.item].y;
-            const int tz = y % I->ntz, rem = y / I->ntz;
-            const int ty = rem % I->nty, ck = rem / I->nty;
-            const int i0 = 1 + ck * now.rg.chunk;
-            const March3 geo{k3TZ * tz, k3TY<T> * ty, i0, min(i0 + now.rg.chunk - 1, I->nb_x)};
+            const Inst3<T> *I = insts + now.it.inst;
+            if (!I->active) {
+                next_item(next, counter);
+                continue;
+            }
+            const int par = I->parity;
+            const March3 geo{k3TZ * now.it.tx, k3TY<T> * now.it.ty, now.it.i0, now.it.i1};
             const bool ok = march3d<T, kF>(S, I->rhoE[par], I->uvw[par], I->rhoE[par ^ 1], I->uvw[par ^ 1], geo, grid,
                                            ph, Tmaps3{}, ring, [&](const Upd3<T> &o) {
                                                if (!state_below(o, ph.ggm1, ph.tlo2))
@@ -495,10 +507,11 @@ __global__ void __launch_bounds__(k3NT<T>, min_blocks3<T>(8)) batch3d(Inst3<T> *
                                            });
             if (!ok) acc.err |= kErrWaitTimeout;
         }
-        Inst3<T> *I = insts + now.inst;
-        const int first = now.rg.first, count = now.rg.count;
-        if (publish_step<k3NT<T>>(acc, parts, now.item, &I->done_items, count, &s_last))
-            finalize_step<k3NT<T>, T, kF>(I, parts + first, count, status ? status + now.inst : nullptr, skip_frac);
+        next_item(next, counter); // (in flight while the item's result is published)
+        Inst3<T> *I = insts + now.it.inst;
+        const int first = now.it.first, count = now.it.count;
+        if (publish_step<k3NT<T>>(acc, parts, now.it.part, &I->done_items, count, &s_last))
+            finalize_step<k3NT<T>, T, kF>(I, parts + first, count, status ? status + now.it.inst : nullptr, skip_frac);
     }
 }
 
@@ -788,7 +801,7 @@ template <class T, int D> class BatchEngine final : public BatchBase {
                 I.rhoE[b] = sl.rhoE[b];
                 I.uv[b] = sl.uvx[b];
             }
-            sl.tiles = I.nstrips;
+            sl.tiles = sl.across = I.nstrips;
         } else {
             I.DtDz = I.dt / I.DZ;
             I.nb_z = (int)nb_z;
@@ -801,6 +814,7 @@ template <class T, int D> class BatchEngine final : public BatchBase {
                 I.uvw[b] = sl.uvx[b];
             }
             sl.tiles = I.ntz * I.nty;
+            sl.across = I.ntz;
         }
         e = cudaMemcpyAsync(insts_ + slot, &I, sizeof I, cudaMemcpyHostToDevice, stream_);
         SlotStatus st0{};
@@ -960,9 +974,17 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     struct Slot {
         bool used = false;
         T *rhoE[2] = {nullptr, nullptr}, *uvx[2] = {nullptr, nullptr};
-        int tiles = 0; // strips (2D) or tiles (3D)
+        int tiles = 0, across = 1; // strips (2D) or tiles (3D) in all, along the fastest axis
         size_t ys = 0, nb[3] = {0, 0, 0};
     };
+
+    // How the instances' rows (planes) are cut into step items: `tail` of them, at least, in
+    // items of at most `rest`, what is before in items of `len`.
+    struct Plan {
+        double tail = 1.0;
+        int len = 1, rest = 1;
+    };
+    static constexpr double kTail = 0.6; // in items of `len` per block
 
     void free_slot(Slot &s)
     {
@@ -979,11 +1001,11 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     {
         if constexpr (D == 2) {
             auto k = fused_ ? batch2d<T, true> : batch2d<T, false>;
-            k<<<blocks_, kStripNT, 0, stream_>>>(insts_, items_, ranges_, nitems_, counter, parts_, status_d_,
+            k<<<blocks_, kStripNT, 0, stream_>>>(insts_, items_, nitems_, counter, parts_, status_d_,
                                                  skip_frac_);
         } else {
             auto k = fused_ ? batch3d<T, true> : batch3d<T, false>;
-            k<<<blocks_, k3NT<T>, smem_, stream_>>>(insts_, items_, ranges_, nitems_, counter, parts_, status_d_,
+            k<<<blocks_, k3NT<T>, smem_, stream_>>>(insts_, items_, nitems_, counter, parts_, status_d_,
                                                    skip_frac_);
         }
     }
@@ -994,31 +1016,51 @@ template <class T, int D> class BatchEngine final : public BatchBase {
                                                                            counter, parts_, status_d_);
     }
 
-    // Rows (planes) per step item, at most: the caller's, or the one with the shortest
-    // estimated step: every item costs its rows and about 3 more (halo rows, start and end), the
-    // resident blocks share them out, and at the end they wait for half an item on average. Long
-    // items suit a set that fills the GPU many times over, short ones a set of a few
-    // instances.
-    int pick_chunk() const
+    // The rows (planes) of an instance's step items: `longs` items of `len`, then items of `rest`.
+    static Chunks split(int rows, const Plan &p)
     {
-        if (chunk_ > 0) return chunk_;
-        int best = 0;
+        const int longs = (int)(rows * (1.0 - p.tail)) / p.len, left = rows - longs * p.len;
+        if (left == 0) return Chunks{longs, p.len, 1, longs};
+        const int n = (left + p.rest - 1) / p.rest;
+        return Chunks{longs, p.len, (left + n - 1) / n, longs + n};
+    }
+
+    // Every item costs its rows and about 3 more (halo rows, start and end), and the resident
+    // blocks share them out. All items alike (the caller's rows, or the candidate): at the end the
+    // blocks wait for half an item on average. Long ones first and short ones last: the blocks
+    // end within a part of a short one, as long as the long ones end well before (kTail). Measured
+    // per run: 24 2D instances of 10.4 M cells, 10 steps FP32 fused, 1105 us in items of 32, 1070 of 32
+    // and 12 rows; 48 instances 1957 and 1893; 12 3D instances of 15.8 M cells, 8 steps FP64, 4480 in
+    // items of 32, 4391 of 64 and 32 planes (items of 12 planes lose more than they even out).
+    Plan pick_plan() const
+    {
+        if (chunk_ > 0) return Plan{1.0, chunk_, chunk_};
+        Plan best;
         double best_cost = 0.0;
-        for (int c : {8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256}) {
-            double work = 0.0;
-            int longest = 0;
-            for (const Slot &s : slots_) {
-                if (!s.used) continue;
-                const int n = ((int)s.nb[0] + c - 1) / c, own = ((int)s.nb[0] + n - 1) / n;
-                work += (double)s.tiles * ((double)s.nb[0] + 3.0 * n);
-                longest = std::max(longest, own);
+        for (int len : {8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256})
+            for (int rest : {0, 8, 12, 16, 24, 32}) {
+                if (2 * rest > len || (D == 3 && rest > 0 && rest < 16)) continue;
+                Plan p{1.0, len, rest ? rest : len};
+                double rows = 0.0;
+                for (const Slot &s : slots_)
+                    if (s.used) rows += (double)s.tiles * (double)s.nb[0];
+                if (rest) p.tail = std::min(1.0, kTail * blocks_ * (len + 3) / rows);
+                double work = 0.0, first = 0.0;
+                int longest = 0;
+                for (const Slot &s : slots_) {
+                    if (!s.used) continue;
+                    const Chunks c = split((int)s.nb[0], p);
+                    work += (double)s.tiles * ((double)s.nb[0] + 3.0 * c.count);
+                    first += (double)s.tiles * c.longs * (len + 3.0);
+                    longest = std::max(longest, c.rest);
+                }
+                double cost = work / blocks_ + 0.5 * (longest + 3);
+                if (rest) cost = std::max(cost, first / blocks_ + len + 3);
+                if (best_cost == 0.0 || cost < best_cost) {
+                    best = p;
+                    best_cost = cost;
+                }
             }
-            const double cost = work / blocks_ + 0.5 * (longest + 3);
-            if (best == 0 || cost < best_cost) {
-                best = c;
-                best_cost = cost;
-            }
-        }
         return best;
     }
 
@@ -1026,31 +1068,31 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     // followed by the conservation sums.
     int rebuild(int nsteps)
     {
-        // step items: each instance's rows in even chunks, the instances with the longest
-        // first, so that the last items to be taken are short ones
-        const int cap = pick_chunk();
-        std::vector<int> order;
+        // step items, the longest first, so that the last ones to be taken are short
+        const Plan plan = pick_plan();
+        std::vector<Item> items;
+        std::vector<int2> sums;
+        int parts = 0;
         for (int i = 0; i < cap_; ++i) {
-            host_ranges_[i] = Range{};
-            if (!slots_[i].used) continue;
-            const int nx = (int)slots_[i].nb[0], n = (nx + cap - 1) / cap;
-            host_ranges_[i].chunk = (nx + n - 1) / n;
-            order.push_back(i);
-        }
-        std::stable_sort(order.begin(), order.end(),
-                         [&](int a, int b) { return host_ranges_[a].chunk > host_ranges_[b].chunk; });
-        std::vector<int2> items, sums;
-        for (int i : order) {
             Range &r = host_ranges_[i];
+            r = Range{};
+            if (!slots_[i].used) continue;
             const Slot &sl = slots_[i];
-            r.first = (int)items.size();
-            r.count = sl.tiles * (((int)sl.nb[0] + r.chunk - 1) / r.chunk);
-            for (int k = 0; k < r.count; ++k) items.push_back(make_int2(i, k));
+            const Chunks c = split((int)sl.nb[0], plan);
+            const int count = sl.tiles * c.count;
+            for (int k = 0; k < count; ++k) {
+                const int t = k % sl.tiles, ck = k / sl.tiles;
+                items.push_back(Item{i, parts + k, t % sl.across, t / sl.across, c.begin(ck),
+                                     std::min(c.begin(ck + 1) - 1, (int)sl.nb[0]), parts, count});
+            }
+            parts += count;
             const size_t cells = sl.nb[0] * sl.nb[1] * (D == 3 ? sl.nb[2] : 1), per = (size_t)kSumNT * kSumCells;
             r.sum_first = (int)sums.size();
             r.sum_count = (int)((cells + per - 1) / per);
             for (int k = 0; k < r.sum_count; ++k) sums.push_back(make_int2(i, k));
         }
+        std::stable_sort(items.begin(), items.end(),
+                         [](const Item &a, const Item &b) { return a.i1 - a.i0 > b.i1 - b.i0; });
         cudaError_t e = cudaStreamSynchronize(stream_);
         const size_t most = std::max(items.size(), sums.size());
         if (e == cudaSuccess && most > items_cap_) {
@@ -1058,15 +1100,15 @@ template <class T, int D> class BatchEngine final : public BatchBase {
             cudaFree(parts_);
             parts_ = nullptr;
             items_cap_ = std::max(most, 2 * items_cap_);
-            e = cudaMalloc(&parts_, (sizeof(ItemPart) + 2 * sizeof(int2)) * items_cap_);
-            items_ = reinterpret_cast<int2 *>(parts_ + items_cap_);
-            sum_list_ = items_ + items_cap_;
+            e = cudaMalloc(&parts_, (sizeof(ItemPart) + sizeof(Item) + sizeof(int2)) * items_cap_);
+            items_ = reinterpret_cast<Item *>(parts_ + items_cap_);
+            sum_list_ = reinterpret_cast<int2 *>(items_ + items_cap_);
             if (e != cudaSuccess) items_cap_ = 0;
         }
         nitems_ = (int)items.size();
         nsums_ = (int)sums.size();
         if (e == cudaSuccess && nitems_ > 0)
-            e = cudaMemcpyAsync(items_, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, stream_);
+            e = cudaMemcpyAsync(items_, items.data(), sizeof(Item) * items.size(), cudaMemcpyHostToDevice, stream_);
         if (e == cudaSuccess && nsums_ > 0)
             e = cudaMemcpyAsync(sum_list_, sums.data(), sizeof(int2) * sums.size(), cudaMemcpyHostToDevice, stream_);
         if (e == cudaSuccess)
@@ -1119,7 +1161,8 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     cudaStream_t stream_ = nullptr;
     Inst *insts_ = nullptr;
     Range *ranges_ = nullptr;
-    int2 *items_ = nullptr, *sum_list_ = nullptr;
+    Item *items_ = nullptr;
+    int2 *sum_list_ = nullptr;
     size_t items_cap_ = 0;
     ItemPart *parts_ = nullptr;
     unsigned *counter_ = nullptr; // one per step of the graph and one for the sums

@@ -208,3 +208,21 @@ def test_batch_speed_skip_never_changes_results(cuda, dim, T):
             assert ra.tobytes() == rb.tobytes() and ua.tobytes() == ub.tobytes()
     with pytest.raises(hb.HydroError):
         Batch(dim, T, capacity=1).set_skip_fraction(-1.0)
+
+
+@pytest.mark.parametrize("T", [np.float64, np.float32])
+@pytest.mark.parametrize("sizes", [[(1, 300), (7, 126), (130, 127), (257, 641), (600, 500), (1201, 253), (901, 1500)],
+                                   [(1, 40, 31), (33, 8, 90), (97, 120, 61), (150, 100, 120), (201, 60, 64)]])
+def test_batch_result_independent_of_items(cuda, T, sizes):
+    """Rows cut in long and short items (chosen for the set) against even items of the
+    caller's: identical bits, time steps and sums."""
+    from hydro_b200.batch import Batch, Blast
+
+    dim, got = len(sizes[0]), []
+    for chunk in (0, 1, 10, 4096):
+        b = Batch(dim, T, chunk=chunk, capacity=len(sizes))
+        slots = [b.add(Blast(nb=nb, max_steps=9)) for nb in sizes]
+        b.run(6)
+        got.append([(b.status(s), [a.tobytes() for a in b.state(s)]) for s in slots])
+        b.close()
+    assert all(g == got[0] for g in got[1:])
