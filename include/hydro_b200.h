@@ -74,8 +74,7 @@ typedef struct hydro_step_info {
     double mass;      /* compensated FP64 sum of the new interior density */
     double max_speed; /* max over interior cells of c_s + |u| (Dt_next = C_min / this) */
     unsigned err;     /* bit 0: non-physical state; bit 1: a bounded wait timed out */
-    int kernel;       /* 1 = strip kernel (rows by TMA, or per-lane cp.async where TMA rejects the
-                         row pitch), 2 = direct kernel */
+    int kernel;       /* 1 = strip kernel, 2 = direct kernel */
 } hydro_step_info_t;
 
 /* Kernel selection for the *_step entry points. AUTO takes the strip kernel whenever the
@@ -200,16 +199,17 @@ unsigned hydro2d_noalloc_launch_shape(size_t NB_X, size_t NB_Y, int strip, int s
  *    9 and 12). Tiles of 8, 12 and 16 rows run one warp per row; a 9-row tile runs on 8
  *    warps, warp 0 holding both halo rows. Built-in: 9, which also runs for arrays that are not
  *    all 16-byte aligned;
- *  chunk: the most rows (2D) or planes (3D) one block marches (built-in 256); blocks take
- *    fewer on grids too small to fill the GPU with that many (sized from the grid and the
- *    SM count);
+ *  chunk: the most rows (2D) or planes (3D) one block marches; blocks take fewer on grids too
+ *    small to fill the GPU with that many. Built-in: up to 256, chosen by a model of the
+ *    launch's time from the grid and the SM count, and in 3D in two lengths where that is
+ *    faster (long chunks first, short ones last);
  *  blocks_per_sm: 2D only, the register budget of the kernel: 4, the built-in one (4
  *    resident blocks per SM in FP64, 7 in FP32), or 5 in FP64 / 8 in FP32.
  * Process-wide; the results do not depend on the shape. No counterpart in the reference,
  * whose single-task kernel has no launch shape. */
 int hydro_set_launch_shape(int dim, int precision_bytes, int warps, int chunk, int blocks_per_sm);
 /* The shape the last strip-kernel step on the current device used (warps: the 3D tile
- * height in rows as above, 0 in 2D), and
+ * height in rows as above, 0 in 2D; chunk: the longer length where there are two), and
  * whether its rows / planes were staged by tensor-map loads (1) or per-lane copies (0). */
 int hydro_last_launch_shape(int *warps, int *chunk, int *blocks_per_sm, int *tma);
 

@@ -136,9 +136,9 @@ def lib():
 
 
 def set_launch_shape(dim: int, dtype, warps: int = 0, chunk: int = 0, blocks: int = 0):
-    """Launch shape of the plain strip kernels for (dim, precision): 3D warps per block
-    (tile rows with halo), rows / planes per block, 2D register budget in blocks per SM
-    (0 = built-in for each). Results do not depend on it."""
+    """Launch shape of the plain strip kernels for (dim, precision): 3D tile rows with halo
+    (built-in 9), the most rows / planes per block, 2D register budget in blocks per SM (0 =
+    built-in for each). Results do not depend on it."""
     _check(lib().hydro_set_launch_shape(int(dim), np.dtype(dtype).itemsize, int(warps), int(chunk), int(blocks)))
 
 

@@ -1,22 +1,24 @@
 """Tile-shape autotuner, keyed on dimensionality and precision.
 
 Plain path (`tune_plain`): the strip kernels take two shape parameters each. Both take the
-most X rows (2D) or planes (3D) one block marches (`chunk`, 0 for the built-in 256; grids
-too small to fill the GPU with such blocks take fewer, so a value tuned on one grid suits
-others): longer chunks re-read fewer halo rows but give fewer blocks. The 3D kernel also
-takes its tile height in rows with the one-row halo: 8, 9, 12 or 16 in FP64, 8 or 16 in
-FP32. Tiles of 8, 12 and 16 rows run one warp per row (taller tiles recompute fewer halo
-rows but hold one block per SM); the 9-row tile runs on 8 warps, warp 0 holding both halo
-rows (FP64 with tensor-map staging). The 2D kernel also takes its register budget in resident
+most X rows (2D) or planes (3D) one block marches (`chunk`, 0 for the built-in choice, which a
+model of the launch's time makes, at most 256; grids too small to fill the GPU with such blocks
+take fewer, so a value tuned on one grid suits others): longer chunks re-read fewer halo rows
+but give fewer blocks. The 3D kernel also takes its tile height in rows with the one-row halo:
+8, 9, 12 or 16 in FP64, 8 or 16 in FP32, 0 for the built-in 9. Tiles of 8, 12 and 16 rows run
+one warp per row (taller tiles recompute fewer halo rows but hold one block per SM); the 9-row
+tile runs on 8 warps, warp 0 holding both halo rows. The 2D kernel also takes its register budget in resident
 blocks per SM (4, or 5 in FP64 / 8 in FP32): more resident warps against fewer registers
 per thread. `tune_plain` times a few steps of the blast on the grid it is given for every
 candidate, keeps the fastest and installs it in the library (hydro_set_launch_shape); the
 results do not depend on the shape.
 
 Batched path (`tune`): the batched kernels take a fixed block shape (2D: 128 lanes over
-126 interior columns; 3D: 8 x 32 lanes over 6 x 30 interior columns) and one free tile
-parameter, the rows (planes) a work item marches, `chunk`. Longer chunks re-read fewer halo rows and take fewer work items; shorter ones
-balance uneven instances better, so the best value depends on how much work a step holds:
+126 interior columns; 3D: 9 rows x 32 columns over 7 x 30 interior cells) and one free tile
+parameter, the rows (planes) a work item marches, `chunk`. Longer chunks re-read fewer halo
+rows and take fewer work items; shorter ones balance uneven instances better, so the best value
+depends on how much work a step holds (without a tuned value the engine chooses long and short
+items for the instances at hand):
 `tune` times a batch drawn like the batched workload in 2D (256 seeded blasts, sides
 log-uniform in [64, 2048]; a smaller batch favours shorter chunks) and 48 seeded 3D blasts
 with sides in [32, 256] in 3D, for each candidate, and keeps the fastest.
@@ -116,7 +118,7 @@ def best_chunk(dim, dtype):
 
 # plain-path candidates per (dim, precision bytes): (3D tile rows with halo or 2D blocks
 # per SM, the other 0) and chunks
-PLAIN_SHAPES = {(2, 4): [(0, 4), (0, 8)], (2, 8): [(0, 4), (0, 5)], (3, 4): [(8, 0), (16, 0)],
+PLAIN_SHAPES = {(2, 4): [(0, 4), (0, 8)], (2, 8): [(0, 4), (0, 5)], (3, 4): [(0, 0), (8, 0), (16, 0)],
                 (3, 8): [(9, 0), (8, 0), (12, 0), (16, 0)]}
 PLAIN_CHUNKS = {2: (0, 32, 64, 128, 256), 3: (0, 16, 32, 64, 128)}
 
