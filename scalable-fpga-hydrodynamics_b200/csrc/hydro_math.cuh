@@ -292,8 +292,9 @@ template <class T> struct Cell2 {
 //
 // Strict: products by 1/2 are exact, so they move into an fma with the sum that follows
 // (E/rho - temp/2, and the 1/2 of the kinetic energy taken off the product r temp instead of
-// off r): the same rounding of the same value, one operation less each. A product so small
-// that 1/2 of it would round lies far below the ulp of the sum it enters.
+// off r): the same rounding of the same value, one operation less each. In the range that
+// `bad` leaves, a product so small that 1/2 of it would round lies below a quarter ulp of the
+// sum it enters, and r temp overflows only where the squared impedance is out of range.
 template <class T, bool kF = false, class PH>
 __device__ __forceinline__ Cell2<T> cell2_fast(T ur, T uu, T uv, T uE, const PH &ph, bool &bad)
 {
@@ -426,8 +427,9 @@ __device__ __forceinline__ Flux2<T> face_flux(const FaceIn<T> &L, const FaceIn<T
         return F2;
     }
     const T us = A::mul(A::half, A::sub(A::add(L.un, R.un), A::mul(diva, A::sub(R.p, L.p))));
-    // 2 p*: its 1/2 is exact and moves into the sums below
-    const T ps2 = A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un)));
+    // (the 1/2 of p* stays a product of its own: moved into the sums below it gives other bits
+    // where a pressure or a flux is subnormal or next to the largest number)
+    const T ps = A::mul(A::half, A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un))));
     const bool up = us >= T(0);
     const T r = up ? L.r : R.r;
     const T mn = up ? L.mn : R.mn;
@@ -437,9 +439,9 @@ __device__ __forceinline__ Flux2<T> face_flux(const FaceIn<T> &L, const FaceIn<T
     // the reference's "+ ZERO" turns -0 into +0: kept where a momentum of -0 would show it,
     // left out where the flux enters the density (never -0 in a cell that has a finite 1/rho)
     F.r = A::mul(r, us);
-    F.n = A::fma(A::half, ps2, A::mul(mn, us));
+    F.n = A::add(A::mul(mn, us), ps);
     F.t = A::add(A::mul(mt, us), T(0));
-    F.E = A::fma(A::half, A::mul(ps2, us), A::mul(e, us));
+    F.E = A::add(A::mul(e, us), A::mul(ps, us));
     return F;
 }
 
@@ -719,7 +721,7 @@ __device__ __forceinline__ Flux3<T> face_flux3(const FaceIn3<T> &L, const FaceIn
         return F3;
     }
     const T us = A::mul(A::half, A::sub(A::add(L.un, R.un), A::mul(diva, A::sub(R.p, L.p))));
-    const T ps2 = A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un))); // 2 p*, as in 2D
+    const T ps = A::mul(A::half, A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un))));
     const bool up = us >= T(0);
     const T r = up ? L.r : R.r;
     const T mn = up ? L.mn : R.mn;
@@ -728,10 +730,10 @@ __device__ __forceinline__ Flux3<T> face_flux3(const FaceIn3<T> &L, const FaceIn
     const T e = up ? L.eup : R.eup;
     Flux3<T> F;
     F.r = A::mul(r, us);
-    F.n = A::fma(A::half, ps2, A::mul(mn, us));
+    F.n = A::add(A::mul(mn, us), ps);
     F.t1 = A::add(A::mul(m1, us), T(0));
     F.t2 = A::add(A::mul(m2, us), T(0));
-    F.E = A::fma(A::half, A::mul(ps2, us), A::mul(e, us));
+    F.E = A::add(A::mul(e, us), A::mul(ps, us));
     return F;
 }
 

@@ -146,7 +146,7 @@ __device__ __forceinline__ Flux3<T> face_from(const Side3<T> &L, const Side3<T> 
         ps = A::mul(A::half, A::fma(-a, A::sub(R.un, L.un), A::add(L.p, R.p)));
     } else {
         us = A::mul(A::half, A::sub(A::add(L.un, R.un), A::mul(diva, A::sub(R.p, L.p))));
-        ps = A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un))); // 2 p*
+        ps = A::mul(A::half, A::sub(A::add(L.p, R.p), A::mul(a, A::sub(R.un, L.un))));
     }
     const bool up = us >= T(0);
     const T r = up ? L.r : R.r;
@@ -165,10 +165,10 @@ __device__ __forceinline__ Flux3<T> face_from(const Side3<T> &L, const Side3<T> 
         F.t2 = A::mul(m2, us);
         F.E = A::fma(e, us, A::mul(ps, us));
     } else {
-        F.n = A::fma(A::half, ps, A::mul(mn, us));
+        F.n = A::add(A::mul(mn, us), ps);
         F.t1 = A::add(A::mul(m1, us), T(0));
         F.t2 = A::add(A::mul(m2, us), T(0));
-        F.E = A::fma(A::half, A::mul(ps, us), A::mul(e, us));
+        F.E = A::add(A::mul(e, us), A::mul(ps, us));
     }
     return F;
 }
