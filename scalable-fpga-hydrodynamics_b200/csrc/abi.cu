@@ -78,11 +78,12 @@ template <class T> __global__ void fused_math_kernel(const T *x, long long n, T 
     }
 }
 
-// The same for the strict conversion's straight-line forms (regular inputs).
+// The same for the strict conversion's straight-line forms (regular inputs; as there, the
+// intrinsic for the reciprocal of a negative FP64 value).
 template <class T> __global__ void strict_math_kernel(const T *x, long long n, T *rcp, T *sq)
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        rcp[i] = Ex<T>::rcp(x[i]);
+        rcp[i] = sizeof(T) == 4 || x[i] > T(0) ? Ex<T>::rcp(x[i]) : Ar<T>::rcp(x[i]);
         sq[i] = Ex<T>::sqrt(x[i]);
     }
 }

@@ -423,6 +423,7 @@ __global__ void __launch_bounds__(kStripNT, Batch2dOcc<T>::value) batch2d(Inst2<
                 s_now.grid = Grid2{I->nb_x, I->nb_y, 1, I->ys};
                 s_now.c = StepConsts<T>(I->ph, I->DtDx, I->DtDy, T(0), (T)I->ggm1,
                                         (T)skip_tlo2(batch_threshold(I, skip_frac)));
+                s_now.c.odd = I->ph.odd && !kF;
             }
         }
         __syncthreads();
@@ -487,6 +488,7 @@ __global__ void __launch_bounds__(k3NT<T>, min_blocks3<T>(8)) batch3d(Inst3<T> *
                 s_now.grid = Grid3(I->nb_x, I->nb_y, I->nb_z, 1);
                 s_now.c = StepConsts<T>(I->ph, I->DtDx, I->DtDy, I->DtDz, (T)I->ggm1,
                                         (T)skip_tlo2(batch_threshold(I, skip_frac)));
+                s_now.c.odd = I->ph.odd && !kF;
             }
         }
         __syncthreads();

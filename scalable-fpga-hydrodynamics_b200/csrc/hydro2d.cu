@@ -329,6 +329,7 @@ int step2d(const T *rhoE, const T *uv, T *rhoE_next, T *uv_next, T *Dt_next, con
     cudaError_t e;
     unsigned nblocks;
     if (use_strip) {
+        g.ph.odd = ph.odd && !fused;
         const int nstrips = (int)((nb_y + kStripW - 1) / kStripW);
         // rows per block: at most the cap (the tuned value when one is set with
         // hydro_set_launch_shape, else 256), at least 2 (one row per block measured no faster)

@@ -287,6 +287,7 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
     g.rhoE = rhoE; g.uvw = uvw; g.rhoE_n = rhoE_next; g.uvw_n = uvw_next; g.Dt_next = Dt_next;
     g.ph = ph; g.DtDx = DtDx; g.DtDy = DtDy; g.DtDz = DtDz;
     g.c = StepConsts<T>(ph, DtDx, DtDy, DtDz);
+    g.c.odd = ph.odd && !fused;
     g.nb_x = (int)nb_x; g.nb_y = (int)nb_y; g.nb_z = (int)nb_z;
     g.zs = (long long)nb_z + 2; g.zy = (long long)(nb_y + 2) * g.zs;
     g.scr = ctx->scr; g.status = ctx->status_d; g.seq = ++ctx->seq;

@@ -148,8 +148,10 @@ template <> struct Fu<float> {
 // The correction's own error is below 2^-53 ulp (reciprocal) and 2^-50 ulp (square root), so
 // only an input whose exact result lies that close to a rounding midpoint could round the
 // wrong way: for the FP64 reciprocal the single significand 2 - 2^-52 (whose start value is
-// rounded away from the tie), for the FP64 square root the few dozen solutions of n 2^54 - q^2 = c and n 2^55 - q^2 = c with small c. The
-// tests enumerate these, and every FP32 significand.
+// rounded away from the tie for a positive argument; K < 0, which makes negative ones, takes
+// the checked conversion: Phys::odd), for the FP64 square root the few dozen solutions of
+// n 2^54 - q^2 = c and n 2^55 - q^2 = c with small c. The tests enumerate these, and every
+// FP32 significand of either sign.
 template <class T> struct Ex;
 
 template <> struct Ex<double> {
@@ -219,13 +221,18 @@ template <class T> __device__ __forceinline__ T smax(T a, T b) { return (a < b) 
 template <class T> struct Phys {
     T C_min, gamma, gm1, divgamma, K;
     T iK;     // 1 / K (fused arithmetic: 1/(K a) = (1/K)(1/a))
-    bool odd; // K or gamma - 1 of no ordinary size: every cell takes the checked conversion
+    // K or gamma - 1 of no ordinary size, or FP64 and K < 0, whose reciprocals Ex::rcp does not
+    // round right: every cell takes the checked conversion. False in launches of fused arithmetic,
+    // whose reciprocals of K a come from 1 / K. (Tested per cell instead, by the
+    // low word of the impedance, K > 0 paid for it: 256 x 256 x 255 FP64 484 -> 519 us, 512^3
+    // 3157 -> 3177.)
+    bool odd;
 
     static Phys make(T C_min, T gamma, T gm1, T divgamma, T K)
     {
         const auto usual = [](T x) { return x > T(1.0 / 1048576) && x < T(1048576); };
         return Phys{C_min, gamma, gm1, divgamma, K, T(1) / K,
-                    !(usual(K < T(0) ? -K : K) && usual(gamma) && usual(gm1) && usual(divgamma))};
+                    !(usual(K < T(0) && sizeof(T) == 4 ? -K : K) && usual(gamma) && usual(gm1) && usual(divgamma))};
     }
 };
 

@@ -95,3 +95,14 @@ def test_fp64_random(cuda):
     _check(cuda, x)
     near = 1.0 + rng.integers(0, 2 ** 20, 500_000) * 2.0 ** -52  # next to 1, 2 and 4
     _check(cuda, np.concatenate([near, 2.0 / near, 4.0 / near]))
+
+
+def test_fp64_hard_cases_negative(cuda):
+    """The reciprocals of negative arguments, which the impedances of K < 0 are."""
+    x = -np.array(_rcp_hard() + [1.0, 2.0, 1.0 + 2 ** -52, 1.5 - 2 ** -52, 4.0 - 2 ** -51])
+    for e in range(-399, 399, 3):
+        r, _ = _device(cuda, x * 2.0 ** e)
+        assert np.array_equal(1.0 / (x * 2.0 ** e), r)
+    rng = np.random.default_rng(8)
+    x = -np.ldexp(rng.uniform(1.0, 2.0, 4_000_000), rng.integers(-400, 400, 4_000_000))
+    assert np.array_equal(1.0 / x, _device(cuda, x)[0])
