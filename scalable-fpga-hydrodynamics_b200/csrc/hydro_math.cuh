@@ -525,24 +525,29 @@ template <class T, bool kF = false, class PH> __device__ __forceinline__ T speed
 // their FP64 pipe for the update), with a relative margin of 2^-12, far above the
 // roundings of the conversions, of this test and of the exact speed's own evaluation, on
 // inputs in ranges where no product overflows or becomes subnormal; anything else (NaN,
-// non-positive rho or E, out of range) answers false and takes the exact path.
+// non-positive rho or E, out of range) answers false and takes the exact path. So does a
+// state whose pressure is not certainly positive (m2 not below 2 E rho by the margin): its
+// speed may be no number, which the exact path flags. (An energy too large for these products
+// makes the left side infinite, and m2 is bounded by it.)
 __device__ __forceinline__ bool speed_below(float r, float E, float m2, float ggm1, float tlo2)
 {
-    if (!(r > 1e-6f) || !(r < 1e6f) || !(E > 1e-6f) || !(E < 1e12f) || !(m2 < 1e24f)) return false;
-    return (ggm1 * E * r + m2) * (2.0f * (1.0f + 1.0f / 4096.0f)) < tlo2 * (r * r);
+    if (!(r > 1e-6f) || !(r < 1e6f) || !(E > 1e-6f)) return false;
+    const float q = E * r;
+    return m2 < q * (2.0f * (1.0f - 1.0f / 4096.0f)) &&
+           (ggm1 * q + m2) * (2.0f * (1.0f + 1.0f / 4096.0f)) < tlo2 * (r * r);
 }
 // The same test in FP64 for FP64 states (no conversions). The ranges are tested on the high
 // words, in integer instructions beside the FP64 pipe's work: at most the ranges above (a
-// value between a bound and the next high word takes the exact path).
+// value between a bound and the next high word takes the exact path), and m2 against 2 E rho
+// (one more in the exponent) less 2^-12 to 2^-13 of it.
 __device__ __forceinline__ bool speed_below(double r, double E, double m2, double ggm1, double tlo2)
 {
     constexpr unsigned lo = 0x3EB0C6F8u;  // the first high word above 1e-6
     constexpr unsigned r_hi = 0x412E8480u; // 1e6
-    constexpr unsigned E_hi = 0x426D1A94u; // 1e12
-    constexpr unsigned m_hi = 0x44EA7843u; // 1e24
-    const bool in = (unsigned)__double2hiint(r) - lo < r_hi - lo && (unsigned)__double2hiint(E) - lo < E_hi - lo &&
-                    (unsigned)__double2hiint(m2) < m_hi;
-    return in && (ggm1 * E * r + m2) * (2.0 * (1.0 + 1.0 / 4096.0)) < tlo2 * (r * r);
+    const double q = E * r;
+    const bool in = __double2hiint(E) >= (int)lo && (unsigned)__double2hiint(r) - lo < r_hi - lo &&
+                    (unsigned)__double2hiint(m2) < (unsigned)__double2hiint(q) + ((1u << 20) - 256u);
+    return in && (ggm1 * q + m2) * (2.0 * (1.0 + 1.0 / 4096.0)) < tlo2 * (r * r);
 }
 // The skip test of a new 2D / 3D state in the state's own precision (S: float, or the constants
 // already in it).
