@@ -307,11 +307,7 @@ int hydro_last_step_info(hydro_step_info_t *info)
     info->max_speed = st.max_speed;
     info->err = st.err;
     info->kernel = c->last_kernel;
-    if (st.err & kErrWaitTimeout) {
-        c->dirty = true;
-        return kErrTimeout;
-    }
-    return (st.err & kErrNonPhysical) ? kErrPhys : kOk;
+    return step_result(st.err, nullptr, &c->dirty);
 }
 
 int hydro_device_contexts(void) { return ctx_count(); }

@@ -237,6 +237,20 @@ int set_launch_shape(int dim, size_t tsize, int warps, int chunk, int blocks)
     return kOk;
 }
 
+int step_result(unsigned err, const char *step, bool *dirty)
+{
+    if (err & kErrWaitTimeout) {
+        *dirty = true;
+        if (step) set_error(kErrTimeout, "%s: a TMA barrier wait timed out", step);
+        return kErrTimeout;
+    }
+    if (err & kErrNonPhysical) {
+        if (step) set_error(kErrPhys, "%s: non-physical state (rho <= 0 or non-finite signal speed)", step);
+        return kErrPhys;
+    }
+    return kOk;
+}
+
 int ctx_count()
 {
     std::lock_guard<std::mutex> lk(g_mu);

@@ -414,16 +414,7 @@ int step2d(const T *rhoE, const T *uv, T *rhoE_next, T *uv_next, T *Dt_next, con
         info->err = st.err;
         info->kernel = (int)(use_strip ? Kernel::Strip : Kernel::Direct);
     }
-    if (st.err & kErrWaitTimeout) {
-        ctx->dirty = true;
-        set_error(kErrTimeout, "step2d: a TMA barrier wait timed out");
-        return kErrTimeout;
-    }
-    if (st.err & kErrNonPhysical) {
-        set_error(kErrPhys, "step2d: non-physical state (rho <= 0 or non-finite signal speed)");
-        return kErrPhys;
-    }
-    return kOk;
+    return step_result(st.err, "step2d", &ctx->dirty);
 }
 
 template <class T>

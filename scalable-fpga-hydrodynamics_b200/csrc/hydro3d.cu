@@ -413,11 +413,7 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
         info->err = st.err;
         info->kernel = (int)(use_strip ? Kernel::Strip : Kernel::Direct);
     }
-    if (st.err & kErrNonPhysical) {
-        set_error(kErrPhys, "step3d: non-physical state (rho <= 0 or non-finite signal speed)");
-        return kErrPhys;
-    }
-    return kOk;
+    return step_result(st.err, "step3d", &ctx->dirty);
 }
 
 template <class T>

@@ -122,6 +122,11 @@ enum : int {
     kErrTimeout = -4,
 };
 
+// Return code of a finished step by the error bits of its record: a time-out (of a wait of the
+// 3D march; the state is then not the step's) before a non-physical state. Latches the error under
+// the step's name when there is one; *dirty: the scratch words must be zeroed before the next step.
+int step_result(unsigned err, const char *step, bool *dirty);
+
 // Encode a 3D tiled tensor map (no swizzle, zero OOB fill). Returns false when the
 // driver entry point is missing or encoding fails.
 bool encode_tmap_3d(CUtensorMap *tm, CUtensorMapDataType dt, const void *base, uint64_t dim0, uint64_t dim1,
