@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(k3NT<T>, min_blocks3<T>(8)) batch3d(Inst3<T> *
     const volatile StepConsts<T> &ph = s_now.c;
     const volatile Grid3 &grid = s_now.grid;
     march3d_init(S);
-    Ring3 ring;
+    Ring<Tile3<T>::NS> ring;
     int next = (int)blockIdx.x; // thread 0: the item to take
     for (;;) {
         __syncthreads(); // everyone is done with the previous item

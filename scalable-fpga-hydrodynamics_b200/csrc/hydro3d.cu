@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(32 * SM::W, min_blocks3<T>(SM::W))
     // (copies: used through references to the parameters, the FP32 forms spilled)
     const Grid3 grid = g.grid;
     const StepConsts<T> c = g.c;
-    Ring3 ring;
+    Ring<SM::NS> ring;
     const bool ok = march3d<T, kF>(S, g.rhoE, g.uvw, g.rhoE_n, g.uvw_n, geo, grid, c, Tmaps3{&tmr, &tmu}, ring, [&](const Upd3<T> &o) {
                                        acc.add_mass(o.r);
                                        if (!state_below(o, ggm1, tlo2))

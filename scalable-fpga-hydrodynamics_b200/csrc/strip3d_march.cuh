@@ -39,6 +39,7 @@
 #pragma once
 
 #include "hydro_rt.cuh"
+#include "ring.h"
 
 namespace hydro {
 
@@ -79,14 +80,6 @@ template <class T, int W_, bool kPair_, Stage3 kStage> struct Smem3 {
         T xFE[32 * (R - 2)];
     } ex[2];
     uint64_t full[NS]; // tensor maps: the stage holds its plane
-};
-
-// A block's place in its ring, kept between marches; every thread holds the same, but for
-// `dead`: a bounded wait of this thread gave up, and it waits no more.
-struct Ring3 {
-    int st = 0;
-    uint32_t phase = 0;
-    bool dead = false;
 };
 
 struct March3 {
@@ -183,7 +176,7 @@ __device__ __forceinline__ Flux3<T> face_from(const Side3<T> &L, const Side3<T> 
 // march runs on without waiting; its values are then not the step's).
 template <class T, bool kF, class SM, class GR, class PH, class Sink>
 __device__ __forceinline__ bool march3d(SM &S, const T *rhoE, const T *uvw, T *rhoE_n, T *uvw_n, const March3 &geo,
-                                             const GR &g, const PH &ph, const Tmaps3 &tm, Ring3 &ring,
+                                             const GR &g, const PH &ph, const Tmaps3 &tm, Ring<SM::NS> &ring,
                                              Sink &&sink)
 {
     using V2 = typename Vec2<T>::type;
@@ -232,7 +225,7 @@ __device__ __forceinline__ bool march3d(SM &S, const T *rhoE, const T *uvw, T *r
     };
     auto issue = [&](int m, int s) {
         if constexpr (SM::kTma) {
-            if (t == 0 && m < nplanes) {
+            if (t == 0 && m < nplanes && !ring.dead) {
                 mbar_arrive_expect_tx(&S.full[s], (uint32_t)(5 * NR * sizeof(T)));
                 tma_load_3d(&S.st[s].r[0][0], tm.r, 2 * geo.kbase, geo.jbase, plane_of(m), &S.full[s]);
                 tma_load_3d(&S.st[s].u[0], tm.u, 3 * geo.kbase, geo.jbase, plane_of(m), &S.full[s]);
@@ -268,16 +261,10 @@ __device__ __forceinline__ bool march3d(SM &S, const T *rhoE, const T *uvw, T *r
     auto wait = [&](int m) {
         if (!SM::kTma || w == 0) issue(m + NS - 1, ring.st == 0 ? NS - 1 : ring.st - 1);
         if constexpr (SM::kTma) {
-            if (!ring.dead && !mbar_wait_bounded(&S.full[ring.st], ring.phase)) ring.dead = true;
+            if (!ring.dead && !mbar_wait_bounded(&S.full[ring.st], ring.phase)) ring.dead = nplanes - m;
         } else {
             cp_async_wait<NS - 1>();
             __syncwarp();
-        }
-    };
-    auto advance = [&]() {
-        if (++ring.st == NS) {
-            ring.st = 0;
-            ring.phase ^= 1u;
         }
     };
     // Row copies: the place within 16 bytes of the first momentum of tile row 0, which runs on
@@ -380,7 +367,7 @@ __device__ __forceinline__ bool march3d(SM &S, const T *rhoE, const T *uvw, T *r
             publish(xc, t, P);
             if (m == 1) fxlo = xface(P);
             __syncthreads();
-            advance();
+            ring.advance();
             swap();
             Pm = keep(P);
             Uu = uu; Uv = uv; Uw = uw; UE = uE;
@@ -424,7 +411,7 @@ __device__ __forceinline__ bool march3d(SM &S, const T *rhoE, const T *uvw, T *r
             const long long zy = g.zy;
             pr += 2 * zy;
             pu += 3 * zy;
-            advance();
+            ring.advance();
             swap();
             fxlo = fxhi;
             Pm = keep(P);
@@ -451,7 +438,7 @@ __device__ __forceinline__ bool march3d(SM &S, const T *rhoE, const T *uvw, T *r
             }
             next_shift(m);
             __syncthreads();
-            advance();
+            ring.advance();
             swap();
             Pm = keep(P);
         }
@@ -467,16 +454,15 @@ __device__ __forceinline__ bool march3d(SM &S, const T *rhoE, const T *uvw, T *r
             next_shift(m);
             publish(xc, t, make_cell3<T, kF>(ur, uu, uv, uw, uE, ph));
             __syncthreads();
-            advance();
+            ring.advance();
             swap();
         }
     }
     if (!SM::kTma) cp_async_wait<0>();
     if (SM::kTma && t == 0 && ring.dead) {
-        // gave up on a stage: wait (bounded) for the loads still in flight before the block's
+        // gave up on a plane: wait (bounded) for the loads still in flight before the block's
         // shared memory is used again or released
-        for (int s = 0; s < NS; ++s)
-            (void)mbar_wait_bounded(&S.full[s], s < ring.st ? ring.phase : ring.phase ^ 1u);
+        ring.drain([&](int s, uint32_t parity) { (void)mbar_wait_bounded(&S.full[s], parity); });
     }
     return !ring.dead;
 }

@@ -1,9 +1,11 @@
-"""Host-side parts of the steps, without a GPU: what a step returns for its error bits."""
+"""Host-side parts of the steps, without a GPU: what a step returns for its error bits, and the
+bookkeeping of the 3D march's ring of stages."""
 from __future__ import annotations
 
 import ctypes
+import subprocess
 
-from conftest import load_pkg
+from conftest import ROOT, load_pkg
 
 hb = load_pkg()
 
@@ -23,3 +25,90 @@ def test_result_of_a_step_by_its_error_bits():
         code, msg = hb.last_error()
         assert (code, bool(word) and word in msg and "step3d" in msg) == (rc, bool(word))
         assert fn(bits, None, ctypes.byref(dirty)) == rc
+
+
+RING = r"""
+#include <cstdio>
+#include <vector>
+#include "ring.h"
+
+// A barrier that one arrival and its bytes complete.
+struct Barrier {
+    int completed = 0;
+    bool pending = false;
+    bool over(uint32_t parity) const { return (uint32_t)(completed & 1) != parity; }
+    void land() { if (pending) { pending = false; ++completed; } }
+};
+
+// Marches of `planes` planes through one ring, as thread 0 runs them; plane `lost` of march `which`
+// never lands while it is waited for. Returns the number of rules broken.
+template <int NS> int run(const std::vector<int> &planes, int which, int lost)
+{
+    hydro::Ring<NS> ring;
+    Barrier bar[NS];
+    int bad = 0;
+    for (int k = 0; k < (int)planes.size(); ++k) {
+        const int n = planes[k];
+        int loads = 0;
+        auto issue = [&](int m, int s) {
+            if (m < n && !ring.dead) {
+                bad += bar[s].pending; // a second arrival within a phase
+                bar[s].pending = true;
+                ++loads;
+            }
+        };
+        for (int m = 0, s = ring.st; m < NS - 1; ++m, s = s + 1 == NS ? 0 : s + 1) issue(m, s);
+        for (int m = 0; m < n; ++m) {
+            issue(m + NS - 1, ring.st == 0 ? NS - 1 : ring.st - 1);
+            if (!ring.dead) {
+                bad += bar[ring.st].over(ring.phase); // the phase of plane m is this one
+                if (k == which && m == lost) {
+                    ring.dead = n - m;
+                } else {
+                    bar[ring.st].land();
+                    bad += !bar[ring.st].over(ring.phase);
+                }
+            }
+            ring.advance();
+        }
+        std::vector<bool> drained(NS, false);
+        ring.drain([&](int s, uint32_t parity) {
+            bad += s < 0 || s >= NS || drained[s] || !bar[s].pending || bar[s].over(parity);
+            drained[s] = true;
+            bar[s].land();
+            bad += !bar[s].over(parity);
+        });
+        for (const Barrier &b : bar) bad += b.pending; // a load in flight behind the march
+        bad += k > which && loads > 0;
+        bad += (ring.dead != 0) != (k >= which);
+    }
+    return bad;
+}
+
+int main()
+{
+    int cases = 0;
+    for (int n0 = 3; n0 < 12; ++n0)
+        for (int n1 = 3; n1 < 12; ++n1)
+            for (int which = 0; which < 4; ++which)
+                for (int lost = 0; lost < (which == 0 ? n0 : which == 1 ? n1 : which == 2 ? 5 : 1); ++lost, ++cases)
+                    if (run<3>({n0, n1, 5}, which, lost) || run<4>({n0, n1, 5}, which, lost)) {
+                        printf("%d %d march %d plane %d\n", n0, n1, which, lost);
+                        return 1;
+                    }
+    printf("%d cases\n", cases);
+    return 0;
+}
+"""
+
+
+def test_ring_after_a_wait_that_gave_up(tmp_path):
+    """A march whose wait for a plane gave up issues no further load (a second arrival within a
+    phase, a load that nothing waits for) and drains exactly those in flight, at every plane, number
+    of planes and place in the ring."""
+    (tmp_path / "ring.cpp").write_text(RING)
+    exe = tmp_path / "ring"
+    csrc = ROOT / "scalable-fpga-hydrodynamics_b200" / "csrc"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(csrc), "-o", str(exe), str(tmp_path / "ring.cpp")], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
