@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <stdio.h>
 #include <string.h>
+#include <utility>
 #include <vector>
 
 #include "../../include/hydro_b200.h"
@@ -75,9 +76,10 @@ struct __align__(16) Item {
     int inst, part, tx, ty, i0, i1, first, count;
 };
 
-// An instance's share of the items of the end-of-run sums.
-struct Range {
-    int sum_first, sum_count;
+// An item of the end-of-run sums: share k of `count` of an instance, the first of which has the
+// slot `first` of the parts.
+struct __align__(16) SumItem {
+    int inst, k, first, count;
 };
 
 struct ItemPart {
@@ -597,8 +599,8 @@ template <int NT, int D, class T, class I> __device__ __forceinline__ void sum_i
 }
 
 template <int NT, int D, class T, class I>
-__global__ void __launch_bounds__(NT) batch_sums(I *insts, const int2 *items, const Range *ranges, int nitems,
-                                                 unsigned *counter, ItemPart *parts, SlotStatus *status)
+__global__ void __launch_bounds__(NT) batch_sums(I *insts, const SumItem *items, int nitems, unsigned *counter,
+                                                 ItemPart *parts, SlotStatus *status)
 {
     __shared__ int s_item;
     __shared__ int s_last;
@@ -612,13 +614,12 @@ __global__ void __launch_bounds__(NT) batch_sums(I *insts, const int2 *items, co
         __syncthreads();
         const int w = s_item;
         if (w >= nitems) break;
-        const int2 it = items[w];
-        I *in = insts + it.x;
+        const SumItem it = items[w];
+        I *in = insts + it.inst;
         BatchAcc acc;
-        const Range rg = ranges[it.x];
-        sum_item<NT, D, T>(in, it.y, rg.sum_count, acc);
-        if (publish_item<NT>(acc, parts, rg.sum_first + it.y, &in->sum_items, rg.sum_count, &s_last))
-            finalize_sums<NT>(in, parts + rg.sum_first, rg.sum_count, status ? status + it.x : nullptr);
+        sum_item<NT, D, T>(in, it.k, it.count, acc);
+        if (publish_item<NT>(acc, parts, it.first + it.k, &in->sum_items, it.count, &s_last))
+            finalize_sums<NT>(in, parts + it.first, it.count, status ? status + it.inst : nullptr);
     }
 }
 
@@ -651,7 +652,6 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         if (own_stream_) e = cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking);
         else stream_ = stream;
         if (e == cudaSuccess) e = cudaMalloc(&insts_, sizeof(Inst) * cap_);
-        if (e == cudaSuccess) e = cudaMalloc(&ranges_, sizeof(Range) * cap_);
         if (e == cudaSuccess) e = cudaMalloc(&counter_, sizeof(unsigned) * counters_);
         if (e == cudaSuccess) e = cudaMalloc(&scratch_bits_, 64);
         if (e == cudaSuccess) e = cudaMemset(scratch_bits_, 0, 64);
@@ -685,7 +685,6 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         }
         sum_blocks_ = nsm * std::max(1, occ_s);
         slots_.resize(cap_);
-        host_ranges_.assign(cap_, Range{});
         *rc = (e == cudaSuccess) ? kOk : kErrCuda;
         if (e != cudaSuccess) set_error(kErrCuda, "batch create: %s", cudaGetErrorString(e));
     }
@@ -697,7 +696,6 @@ template <class T, int D> class BatchEngine final : public BatchBase {
             if (s.used) free_slot(s);
         cudaStreamSynchronize(stream_);
         cudaFree(insts_);
-        cudaFree(ranges_);
         cudaFree(counter_);
         cudaFree(scratch_bits_);
         cudaFree(parts_);
@@ -1014,8 +1012,8 @@ template <class T, int D> class BatchEngine final : public BatchBase {
 
     void launch_sums(unsigned *counter)
     {
-        batch_sums<kSumNT, D, T, Inst><<<sum_blocks_, kSumNT, 0, stream_>>>(insts_, sum_list_, ranges_, nsums_,
-                                                                           counter, parts_, status_d_);
+        batch_sums<kSumNT, D, T, Inst><<<sum_blocks_, kSumNT, 0, stream_>>>(insts_, sum_list_, nsums_, counter, parts_,
+                                                                           status_d_);
     }
 
     // The rows (planes) of an instance's step items: `longs` items of `len`, then items of `rest`.
@@ -1037,32 +1035,53 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     Plan pick_plan() const
     {
         if (chunk_ > 0) return Plan{1.0, chunk_, chunk_};
-        Plan best;
-        double best_cost = 0.0;
+        double rows = 0.0, most = 0.0;
+        for (int i : live_) {
+            rows += (double)slots_[i].tiles * (double)slots_[i].nb[0];
+            most = std::max(most, (double)slots_[i].nb[0]);
+        }
+        // The candidates in the order of what they cost at least, with rows cut without a remainder:
+        // the set is gone through for the first few, until none left can be the best. (Preparing a run
+        // of 256 2D instances took 390 us with all of them and every item sorted, now 205; of two equal
+        // ones the one of shorter items.)
+        struct Candidate {
+            double least;
+            Plan p;
+        };
+        Candidate cand[11 * 6];
+        int n = 0;
         for (int len : {8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256})
             for (int rest : {0, 8, 12, 16, 24, 32}) {
                 if (2 * rest > len || (D == 3 && rest > 0 && rest < 16)) continue;
                 Plan p{1.0, len, rest ? rest : len};
-                double rows = 0.0;
-                for (const Slot &s : slots_)
-                    if (s.used) rows += (double)s.tiles * (double)s.nb[0];
                 if (rest) p.tail = std::min(1.0, kTail * blocks_ * (len + 3) / rows);
-                double work = 0.0, first = 0.0;
-                int longest = 0;
-                for (const Slot &s : slots_) {
-                    if (!s.used) continue;
-                    const Chunks c = split((int)s.nb[0], p);
-                    work += (double)s.tiles * ((double)s.nb[0] + 3.0 * c.count);
-                    first += (double)s.tiles * c.longs * (len + 3.0);
-                    longest = std::max(longest, c.rest);
-                }
-                double cost = work / blocks_ + 0.5 * (longest + 3);
-                if (rest) cost = std::max(cost, first / blocks_ + len + 3);
-                if (best_cost == 0.0 || cost < best_cost) {
-                    best = p;
-                    best_cost = cost;
-                }
+                const double end = p.tail * most;
+                const double least = rows * (1.0 + 3.0 * ((1.0 - p.tail) / len + p.tail / p.rest)) / blocks_ +
+                                     0.5 * (p.rest * end / (p.rest + end) + 3);
+                cand[n++] = Candidate{std::max(least, rest ? len + 3.0 : 0.0), p};
             }
+        std::stable_sort(cand, cand + n, [](const Candidate &a, const Candidate &b) { return a.least < b.least; });
+        Plan best;
+        double best_cost = 0.0;
+        for (int k = 0; k < n && (best_cost == 0.0 || cand[k].least <= best_cost); ++k) {
+            const Plan &p = cand[k].p;
+            double work = 0.0, first = 0.0;
+            int longest = 0;
+            for (int i : live_) {
+                const Slot &s = slots_[i];
+                const Chunks c = split((int)s.nb[0], p);
+                work += (double)s.tiles * ((double)s.nb[0] + 3.0 * c.count);
+                first += (double)s.tiles * c.longs * (p.len + 3.0);
+                longest = std::max(longest, c.rest);
+            }
+            double cost = work / blocks_ + 0.5 * (longest + 3);
+            if (p.rest != p.len) cost = std::max(cost, first / blocks_ + p.len + 3);
+            if (best_cost == 0.0 || cost < best_cost ||
+                (cost == best_cost && std::make_pair(p.len, p.rest) < std::make_pair(best.len, best.rest))) {
+                best = p;
+                best_cost = cost;
+            }
+        }
         return best;
     }
 
@@ -1070,52 +1089,73 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     // followed by the conservation sums.
     int rebuild(int nsteps)
     {
-        // step items, the longest first, so that the last ones to be taken are short
+        live_.clear();
+        for (int i = 0; i < cap_; ++i)
+            if (slots_[i].used) live_.push_back(i);
+        // step items, the longest first, so that the last ones to be taken are short: runs of chunks
+        // of one instance and one length are put in order, and their items written out
+        struct Run {
+            int slot, ck, n, rows, part, count; // chunks ck .. ck + n - 1 of `rows` each
+        };
         const Plan plan = pick_plan();
-        std::vector<Item> items;
-        std::vector<int2> sums;
-        int parts = 0;
-        for (int i = 0; i < cap_; ++i) {
-            Range &r = host_ranges_[i];
-            r = Range{};
-            if (!slots_[i].used) continue;
+        std::vector<Run> runs;
+        size_t parts = 0, nsums = 0;
+        auto sum_count = [](const Slot &sl) {
+            const size_t cells = sl.nb[0] * sl.nb[1] * (D == 3 ? sl.nb[2] : 1), per = (size_t)kSumNT * kSumCells;
+            return (cells + per - 1) / per;
+        };
+        for (int i : live_) {
             const Slot &sl = slots_[i];
             const Chunks c = split((int)sl.nb[0], plan);
-            const int count = sl.tiles * c.count;
-            for (int k = 0; k < count; ++k) {
-                const int t = k % sl.tiles, ck = k / sl.tiles;
-                items.push_back(Item{i, parts + k, t % sl.across, t / sl.across, c.begin(ck),
-                                     std::min(c.begin(ck + 1) - 1, (int)sl.nb[0]), parts, count});
-            }
-            parts += count;
-            const size_t cells = sl.nb[0] * sl.nb[1] * (D == 3 ? sl.nb[2] : 1), per = (size_t)kSumNT * kSumCells;
-            r.sum_first = (int)sums.size();
-            r.sum_count = (int)((cells + per - 1) / per);
-            for (int k = 0; k < r.sum_count; ++k) sums.push_back(make_int2(i, k));
+            const int count = sl.tiles * c.count, whole = c.count - 1 - c.longs; // (and the last chunk)
+            const int last = (int)sl.nb[0] - c.begin(c.count - 1) + 1;
+            if (c.longs > 0) runs.push_back(Run{i, 0, std::min(c.longs, c.count), c.len, (int)parts, count});
+            if (whole > 0) runs.push_back(Run{i, c.longs, whole, c.rest, (int)parts, count});
+            if (c.count > c.longs) runs.push_back(Run{i, c.count - 1, 1, last, (int)parts, count});
+            parts += (size_t)count;
+            nsums += sum_count(sl);
         }
-        std::stable_sort(items.begin(), items.end(),
-                         [](const Item &a, const Item &b) { return a.i1 - a.i0 > b.i1 - b.i0; });
+        std::stable_sort(runs.begin(), runs.end(), [](const Run &a, const Run &b) { return a.rows > b.rows; });
+        // the step items and behind them those of the sums, to the device in one copy
+        std::vector<unsigned char> lists(parts * sizeof(Item) + nsums * sizeof(SumItem));
+        Item *item = reinterpret_cast<Item *>(lists.data());
+        for (const Run &r : runs) {
+            const Slot &sl = slots_[r.slot];
+            const Chunks c = split((int)sl.nb[0], plan);
+            for (int k = r.ck; k < r.ck + r.n; ++k)
+                for (int t = 0, tx = 0, ty = 0; t < sl.tiles; ++t) {
+                    const int i0 = c.begin(k);
+                    *item++ = Item{r.slot, r.part + k * sl.tiles + t, tx, ty, i0, i0 + r.rows - 1, r.part, r.count};
+                    if (++tx == sl.across) {
+                        tx = 0;
+                        ++ty;
+                    }
+                }
+        }
+        SumItem *sum = reinterpret_cast<SumItem *>(item);
+        int first = 0;
+        for (int i : live_) {
+            const int count = (int)sum_count(slots_[i]);
+            for (int k = 0; k < count; ++k) *sum++ = SumItem{i, k, first, count};
+            first += count;
+        }
         cudaError_t e = cudaStreamSynchronize(stream_);
-        const size_t most = std::max(items.size(), sums.size());
-        if (e == cudaSuccess && most > items_cap_) {
-            // one allocation: the parts, the step items, the items of the sums
+        // one allocation: the parts (of the items of a step, or of the sums), the lists
+        const size_t at = sizeof(ItemPart) * std::max(parts, nsums), need = at + lists.size();
+        if (e == cudaSuccess && need > room_) {
             cudaFree(parts_);
             parts_ = nullptr;
-            items_cap_ = std::max(most, 2 * items_cap_);
-            e = cudaMalloc(&parts_, (sizeof(ItemPart) + sizeof(Item) + sizeof(int2)) * items_cap_);
-            items_ = reinterpret_cast<Item *>(parts_ + items_cap_);
-            sum_list_ = reinterpret_cast<int2 *>(items_ + items_cap_);
-            if (e != cudaSuccess) items_cap_ = 0;
+            room_ = std::max(need, 2 * room_);
+            e = cudaMalloc(&parts_, room_);
+            if (e != cudaSuccess) room_ = 0;
         }
-        nitems_ = (int)items.size();
-        nsums_ = (int)sums.size();
-        if (e == cudaSuccess && nitems_ > 0)
-            e = cudaMemcpyAsync(items_, items.data(), sizeof(Item) * items.size(), cudaMemcpyHostToDevice, stream_);
-        if (e == cudaSuccess && nsums_ > 0)
-            e = cudaMemcpyAsync(sum_list_, sums.data(), sizeof(int2) * sums.size(), cudaMemcpyHostToDevice, stream_);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(ranges_, host_ranges_.data(), sizeof(Range) * cap_, cudaMemcpyHostToDevice, stream_);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+        nitems_ = (int)parts;
+        nsums_ = (int)nsums;
+        if (e == cudaSuccess && nitems_ > 0) {
+            items_ = reinterpret_cast<Item *>(reinterpret_cast<unsigned char *>(parts_) + at);
+            sum_list_ = reinterpret_cast<SumItem *>(items_ + parts);
+            e = cudaMemcpyAsync(items_, lists.data(), lists.size(), cudaMemcpyHostToDevice, stream_);
+        }
         if (graph_) {
             cudaGraphExecDestroy(graph_);
             graph_ = nullptr;
@@ -1147,6 +1187,9 @@ template <class T, int D> class BatchEngine final : public BatchBase {
             if (e == cudaSuccess) e = cudaGraphInstantiate(&graph_, g, 0);
             if (g) cudaGraphDestroy(g);
         }
+        // the copy reads the lists: on its way while the graph was made
+        const cudaError_t e3 = cudaStreamSynchronize(stream_);
+        if (e == cudaSuccess) e = e3;
         if (e != cudaSuccess) {
             set_error(kErrCuda, "batch rebuild: %s", cudaGetErrorString(e));
             return kErrCuda;
@@ -1162,17 +1205,16 @@ template <class T, int D> class BatchEngine final : public BatchBase {
     bool own_stream_ = false, dirty_ = true;
     cudaStream_t stream_ = nullptr;
     Inst *insts_ = nullptr;
-    Range *ranges_ = nullptr;
     Item *items_ = nullptr;
-    int2 *sum_list_ = nullptr;
-    size_t items_cap_ = 0;
+    SumItem *sum_list_ = nullptr;
+    size_t room_ = 0; // bytes allocated at parts_
     ItemPart *parts_ = nullptr;
     unsigned *counter_ = nullptr; // one per step of the graph and one for the sums
     size_t counters_ = 256;
     unsigned long long *scratch_bits_ = nullptr;
     SlotStatus *status_h_ = nullptr, *status_d_ = nullptr;
     std::vector<Slot> slots_;
-    std::vector<Range> host_ranges_;
+    std::vector<int> live_; // the slots in use, as of the last rebuild
     int nitems_ = 0, nsums_ = 0, blocks_ = 1, sum_blocks_ = 1, graph_steps_ = -1, smem_ = 0;
     cudaGraphExec_t graph_ = nullptr;
 };

@@ -226,3 +226,28 @@ def test_batch_result_independent_of_items(cuda, T, sizes):
         got.append([(b.status(s), [a.tobytes() for a in b.state(s)]) for s in slots])
         b.close()
     assert all(g == got[0] for g in got[1:])
+
+
+def test_prepare_does_not_pay_for_empty_slots(cuda):
+    """Preparing a run goes by the instances, not by the capacity (65536 slots took 50 times the
+    8 that are in use)."""
+    import time
+
+    from hydro_b200.batch import Batch, Blast
+
+    def prepare(capacity):
+        b = Batch(2, np.float32, capacity=capacity)
+        for k in range(8):
+            b.add(Blast((100 + 7 * k, 90 + 5 * k)))
+        b.prepare(4)
+        best = float("inf")
+        for _ in range(10):
+            b.set_skip_fraction(0.9)  # (what was prepared no longer holds)
+            b.sync()
+            t0 = time.perf_counter()
+            b.prepare(4)
+            best = min(best, time.perf_counter() - t0)
+        b.close()
+        return best
+
+    assert prepare(65536) < 10 * prepare(8)
