@@ -76,3 +76,18 @@ def test_long_and_short_chunks(cuda, oracle, nb, T, chunk):
     _run(cuda, oracle, nb, T, 0, False)
     if chunk and T is np.float64:
         assert hb.last_launch_shape()["chunk"] == chunk
+
+
+@pytest.mark.parametrize("T, nb", [(np.float32, (203, 197, 199)), (np.float32, (221, 150, 148)),
+                                   (np.float64, (170, 170, 170)), (np.float64, (203, 151, 149))])
+def test_two_lengths_and_a_ragged_end(cuda, oracle, T, nb):
+    """Grids whose columns are split in long and short chunks with a shorter last one, by tensor maps
+    and by row copies, in both precisions."""
+    from test_march_host import march_chunks
+
+    tiles = -(-nb[1] // 7) * -(-nb[2] // 30)
+    c = march_chunks(nb[0], tiles, 2 if T is np.float64 else 3)
+    assert c.longs > 0 and 0 < nb[0] - c.begin(c.count - 1) + 1 < c.rest
+    _run(cuda, oracle, nb, T, 0, False)
+    shape = hb.last_launch_shape()
+    assert shape["chunk"] == c.len and shape["tma"] == (T is np.float64 and nb[2] % 2 == 0)

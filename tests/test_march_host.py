@@ -1,8 +1,9 @@
 """Host-side parts of the steps, without a GPU: what a step returns for its error bits, and the
-bookkeeping of the 3D march's ring of stages."""
+bookkeeping of the 3D march's ring of stages, and the split of its planes."""
 from __future__ import annotations
 
 import ctypes
+import random
 import subprocess
 
 from conftest import ROOT, load_pkg
@@ -112,3 +113,39 @@ def test_ring_after_a_wait_that_gave_up(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(csrc), "-o", str(exe), str(tmp_path / "ring.cpp")], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+class Chunks(ctypes.Structure):
+    _fields_ = [("longs", ctypes.c_int), ("len", ctypes.c_int), ("rest", ctypes.c_int), ("count", ctypes.c_int)]
+
+    def begin(self, k):
+        return 1 + (k * self.len if k < self.longs else self.longs * self.len + (k - self.longs) * self.rest)
+
+
+def march_chunks(rows, tiles, per_sm, cap=0, least=3):
+    """How the 3D step splits `rows` planes over `tiles` columns of blocks (csrc/context.cu)."""
+    fn = hb.lib()["_ZN5hydro12march_chunksEmmiii"]
+    fn.argtypes = [ctypes.c_size_t, ctypes.c_size_t] + [ctypes.c_int] * 3
+    fn.restype = Chunks
+    return fn(rows, tiles, per_sm, cap, least)
+
+
+def test_chunks_cover_every_plane_once():
+    """Long chunks and short ones, any numbers: each plane belongs to one chunk, none is empty, at most
+    65535 of them, and an asked-for chunk length is not exceeded."""
+    two = ragged = 0
+    rng = random.Random(3)
+    for _ in range(4000):
+        rows = max(1, int(10 ** rng.uniform(0, 4.5)))
+        tiles = max(1, int(10 ** rng.uniform(0, 4)))
+        cap = rng.choice([0, 0, 0, 1, 2, 7, 64, 300])
+        # (without a GPU the model sees one SM: the resident blocks of 148 asked for in its place)
+        c = march_chunks(rows, tiles, rng.choice([1, 2, 3, 222, 296, 444]), cap, rng.choice([2, 3]))
+        ends = [min(c.begin(k + 1) - 1, rows) for k in range(c.count)]
+        assert 1 <= c.count <= 65535 and c.begin(0) == 1 and ends[-1] == rows, (rows, tiles, cap)
+        assert all(c.begin(k) <= ends[k] for k in range(c.count)), (rows, tiles, cap)
+        assert all(ends[k] + 1 == c.begin(k + 1) for k in range(c.count - 1)), (rows, tiles, cap)
+        assert cap == 0 or (c.longs == 0 and c.rest <= cap)
+        two += c.longs > 0
+        ragged += c.longs > 0 and rows - c.begin(c.count - 1) + 1 < c.rest
+    assert two > 100 and ragged > 50
