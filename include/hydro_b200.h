@@ -73,7 +73,7 @@ typedef struct hydro_queue {
 typedef struct hydro_step_info {
     double mass;      /* compensated FP64 sum of the new interior density */
     double max_speed; /* max over interior cells of c_s + |u| (Dt_next = C_min / this) */
-    unsigned err;     /* bit 0: non-physical state; bit 1: a bounded wait timed out */
+    unsigned err;     /* bit 0: non-physical state; bit 1: a bounded wait of a 3D step timed out */
     int kernel;       /* 1 = strip kernel, 2 = direct kernel */
 } hydro_step_info_t;
 
@@ -182,8 +182,7 @@ int hydro2d_step_f64_noalloc(const double *d_rhoE, const double *d_uv, double *d
 
 /* Results of the last hydro2d_step_f64_noalloc call in the current CUDA context, read from
  * the fixed array without allocating: the copy is ordered on `stream` (the step's stream),
- * which it synchronises. Returns HYDRO_OK, HYDRO_ERR_NONPHYSICAL or HYDRO_ERR_TIMEOUT from
- * the step's error bits. No counterpart in the reference. */
+ * which it synchronises. Returns HYDRO_OK or HYDRO_ERR_NONPHYSICAL from the step's error bits. No counterpart in the reference. */
 int hydro2d_noalloc_last_info(void *stream, hydro_step_info_t *info);
 
 /* The launch shape hydro2d_step_f64_noalloc uses on a GPU with `sms` multiprocessors, for
@@ -197,8 +196,8 @@ unsigned hydro2d_noalloc_launch_shape(size_t NB_X, size_t NB_Y, int strip, int s
  * autotuner picks it. 0 keeps the built-in choice for any field.
  *  warps: 3D only, the tile height in rows with the one-row halo (8, 16, and in FP64 also
  *    9 and 12). Tiles of 8, 12 and 16 rows run one warp per row; a 9-row tile runs on 8
- *    warps, warp 0 holding both halo rows. Built-in: 9, which also runs for arrays that are not
- *    all 16-byte aligned;
+ *    warps, warp 0 holding both halo rows. Built-in: 9 in both precisions (in FP32 asked for
+ *    by 0 only), which also runs for arrays that are not all 16-byte aligned;
  *  chunk: the most rows (2D) or planes (3D) one block marches; blocks take fewer on grids too
  *    small to fill the GPU with that many. Built-in: up to 256, chosen by a model of the
  *    launch's time from the grid and the SM count, and in 3D in two lengths where that is

@@ -368,8 +368,8 @@ def alloc_state(nb, dtype, device="cuda"):
 
 class BlastRun:
     """The reference's host loop for one rank and one subdomain covering the domain
-    (hydro2d/main.cxx:686-815): state stays on the device; each step reads the new Dt
-    back (the only per-step device-to-host copy the loop needs)."""
+    (hydro2d/main.cxx:686-815): state stays on the device; the new Dt comes with the record
+    of each step, in host-mapped memory."""
 
     def __init__(self, nb, dtype=np.float64, kernel=KERNEL_AUTO, stream=None, blast=None, arith=None):
         """`blast` (a hydro_b200.batch.Blast) overrides the reference's initial condition

@@ -49,7 +49,7 @@ template <class T> struct alignas(128) Inst2 {
     unsigned sum_items; // items of the end-of-run conservation sums done
     long long ys;
     long long steps, max_steps;
-    int nb_x, nb_y, nstrips;
+    int nb_x, nb_y;
     int parity, active;
     unsigned done_items, err;
 };
@@ -65,7 +65,7 @@ template <class T> struct alignas(128) Inst3 {
     unsigned sum_items; // items of the end-of-run conservation sums done
     long long zs, zy;
     long long steps, max_steps;
-    int nb_x, nb_y, nb_z, ntz, nty;
+    int nb_x, nb_y, nb_z;
     int parity, active;
     unsigned done_items, err;
 };
@@ -796,25 +796,22 @@ template <class T, int D> class BatchEngine final : public BatchBase {
         I.active = (0.0 < s.t_end) && (0 < s.max_steps);
         if constexpr (D == 2) {
             I.ys = (long long)ys;
-            I.nstrips = (int)((nb_y + kStripW - 1) / kStripW);
             for (int b = 0; b < 2; ++b) {
                 I.rhoE[b] = sl.rhoE[b];
                 I.uv[b] = sl.uvx[b];
             }
-            sl.tiles = sl.across = I.nstrips;
+            sl.tiles = sl.across = (int)((nb_y + kStripW - 1) / kStripW);
         } else {
             I.DtDz = I.dt / I.DZ;
             I.nb_z = (int)nb_z;
             I.zs = (long long)nb_z + 2;
             I.zy = (long long)(nb_y + 2) * I.zs;
-            I.ntz = (int)((nb_z + k3TZ - 1) / k3TZ);
-            I.nty = (int)((nb_y + k3TY<T> - 1) / k3TY<T>);
             for (int b = 0; b < 2; ++b) {
                 I.rhoE[b] = sl.rhoE[b];
                 I.uvw[b] = sl.uvx[b];
             }
-            sl.tiles = I.ntz * I.nty;
-            sl.across = I.ntz;
+            sl.across = (int)((nb_z + k3TZ - 1) / k3TZ);
+            sl.tiles = sl.across * (int)((nb_y + k3TY<T> - 1) / k3TY<T>);
         }
         e = cudaMemcpyAsync(insts_ + slot, &I, sizeof I, cudaMemcpyHostToDevice, stream_);
         SlotStatus st0{};

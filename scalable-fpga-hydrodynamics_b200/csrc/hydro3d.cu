@@ -245,9 +245,6 @@ __global__ void init3d_kernel(T *rhoE, T *uvw, int nb_x, int nb_y, int nb_z, lon
 
 // ----------------------------------------------------------------- host drivers ---
 namespace {
-template <class T> CUtensorMapDataType tmap_type3();
-template <> CUtensorMapDataType tmap_type3<double>() { return CU_TENSOR_MAP_DATA_TYPE_FLOAT64; }
-template <> CUtensorMapDataType tmap_type3<float>() { return CU_TENSOR_MAP_DATA_TYPE_FLOAT32; }
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) % 16) == 0; }
 } // namespace
 
@@ -334,9 +331,9 @@ int step3d(const T *rhoE, const T *uvw, T *rhoE_next, T *uvw_next, T *Dt_next, c
         std::memset(&tmu, 0, sizeof tmu);
         if (tma) {
             const uint64_t zs = nb_z + 2, ys = nb_y + 2, xs = nb_x + 2;
-            if (!encode_tmap_3d(&tmr, tmap_type3<T>(), rhoE, 2 * zs, ys, xs, 2 * zs * sizeof(T), 2 * zs * ys * sizeof(T),
+            if (!encode_tmap_3d(&tmr, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, rhoE, 2 * zs, ys, xs, 2 * zs * sizeof(T), 2 * zs * ys * sizeof(T),
                                 64, (uint32_t)rows, 1) ||
-                !encode_tmap_3d(&tmu, tmap_type3<T>(), uvw, 3 * zs, ys, xs, 3 * zs * sizeof(T), 3 * zs * ys * sizeof(T),
+                !encode_tmap_3d(&tmu, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, uvw, 3 * zs, ys, xs, 3 * zs * sizeof(T), 3 * zs * ys * sizeof(T),
                                 96, (uint32_t)rows, 1)) {
                 set_error(kErrCuda, "step3d: tensor maps rejected");
                 return kErrCuda;

@@ -15,7 +15,7 @@ namespace hydro {
 // Which kernel a step runs.
 enum class Kernel : int {
     Auto = 0,   // strip kernel when its alignment rules hold, else the direct kernel
-    Strip = 1,  // TMA-fed strip march (faces computed once)
+    Strip = 1,  // strip march (faces computed once)
     Direct = 2, // one thread per cell, neighbours loaded directly (faces computed twice)
 };
 
@@ -31,7 +31,7 @@ struct DevCtx {
     int last_warps = 0;  // its launch shape (strip kernels): warps per block, rows/planes per block
     int last_chunk = 0;
     int last_blocks = 0;   // 2D: its register budget in blocks per SM
-    bool last_tma = false; // its rows/planes staged by tensor-map loads
+    bool last_tma = false; // 3D: its planes staged by tensor-map loads
     bool dirty = false; // a launch failed: scratch words must be re-zeroed
 };
 
