@@ -55,26 +55,31 @@ struct StepStatus {
     unsigned int pad;
 };
 
-// Skip threshold of a step: the previous max of the same problem, scaled.
+// Skip threshold of a step: the previous max of the same problem, scaled. Plain loads: nobody
+// writes the history before every block of the launch has read it, so an SM's later blocks find
+// it in L1.
 __device__ __forceinline__ double skip_threshold(const StepScratch *scr, unsigned long long key)
 {
-    const unsigned long long k = *reinterpret_cast<const volatile unsigned long long *>(&scr->hist_key);
-    const double m = *reinterpret_cast<const volatile double *>(&scr->hist_max);
-    return (key != 0ull && k == key) ? kSkipFrac * m : 0.0;
+    return (key != 0ull && scr->hist_key == key) ? kSkipFrac * scr->hist_max : 0.0;
 }
 
 // The thresholds of one block: `hist` from the previous step, checked against this step's max
-// at its end, and `f` for the skip test, raised to the max that the launch's finished blocks
-// have reached so far: a cell below that cannot hold the max, whatever the history says. Both
-// rounded down to float, so that every skipped cell is provably below the value in double.
+// at its end, and `f` for the skip test: without a history the max that the launch's finished
+// blocks have reached so far, below which a cell cannot hold the max either. Both rounded down to
+// float, so that every skipped cell is provably below the value in double. (The running max lies
+// where all blocks put theirs by atomics, and so many loads of one place queue up in L2: read by
+// every warp of every launch, with the history volatile too, 1 x 1000000 FP64, blocks of one row,
+// took 133 us.)
 struct SkipLimits {
     float hist, f;
 };
 __device__ __forceinline__ SkipLimits skip_limits(const StepScratch *scr, unsigned long long key)
 {
-    const unsigned long long m = *reinterpret_cast<const volatile unsigned long long *>(&scr->max_bits);
-    const double h = skip_threshold(scr, key), now = __longlong_as_double((long long)m);
-    return SkipLimits{__double2float_rd(h), __double2float_rd(h > now ? h : now)};
+    const double h = skip_threshold(scr, key);
+    double f = h;
+    if (h == 0.0)
+        f = __longlong_as_double((long long)*reinterpret_cast<const volatile unsigned long long *>(&scr->max_bits));
+    return SkipLimits{__double2float_rd(h), __double2float_rd(f)};
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
