@@ -61,7 +61,7 @@ template <class T> __device__ __forceinline__ Cell2<T> load_cell2(const Args2<T>
     return make_cell2<T>(g.rhoE[2 * c], g.uv[2 * c], g.uv[2 * c + 1], g.rhoE[2 * c + 1], g.ph);
 }
 
-template <class T> __global__ void __launch_bounds__(kDirectNT) direct2d(Args2<T> g)
+template <class T> __global__ void __launch_bounds__(kDirectNT, sizeof(T) == 8 ? 5 : 1) direct2d(Args2<T> g)
 {
     StepAcc acc;
     const int j = 1 + blockIdx.x * kDirectNT + threadIdx.x;
