@@ -119,7 +119,8 @@ template <class T, bool kF, int kMinB> __global__ void __launch_bounds__(kStripN
     const float tlo2 = skip_tlo2(lim.f), ggm1 = g.ggm1;
     const Grid2 grid{g.nb_x, g.nb_y, g.xwrap, g.ys};
     const StepConsts<T> c(g.ph, g.DtDx, g.DtDy, T(0));
-    march2d<T, kF>(S, g.rhoE, g.uv, g.rhoE_n, g.uv_n, geo, grid, c, [&](const Upd2<T> &o) {
+    constexpr int kUnroll = sizeof(T) == 8 && kMinB > 4 ? 1 : 2;
+    march2d<T, kF, kUnroll>(S, g.rhoE, g.uv, g.rhoE_n, g.uv_n, geo, grid, c, [&](const Upd2<T> &o) {
         acc.add_mass(o.r);
         if (!state_below(o, ggm1, tlo2)) acc.add_speed(o.r, speed2<T, kF>(o.r, o.u, o.v, o.E, c));
     });

@@ -72,8 +72,10 @@ struct Grid2 {
 // FP64; columns two to a lane, loaded straight to registers, 59 against 79 at 8000 x 8000; strips
 // of one warp, which need no block barrier, 75.)
 //
-// kF: fused arithmetic (hydro_math.cuh).
-template <class T, bool kF, class GR, class PH, class Sink>
+// kF: fused arithmetic (hydro_math.cuh). kUnroll: rows per turn of the loop; two need more than the
+// 96 registers of 5 blocks per SM in FP64 (8000 x 8000 fused 1469 us with the spills, 920 one at a
+// time; strict 1127 and 848; 738 and 784 with two rows and 4 blocks, the built-in form).
+template <class T, bool kF, int kUnroll = 2, class GR, class PH, class Sink>
 __device__ __forceinline__ void march2d(Smem2<T> &S, const T *rhoE, const T *uv, T *rhoE_n, T *uv_n, const March2 &geo,
                                         const GR &g, const PH &ph, Sink &&sink)
 {
@@ -143,7 +145,7 @@ __device__ __forceinline__ void march2d(Smem2<T> &S, const T *rhoE, const T *uv,
         Pm = P;
         Ur = a.x; Uu = b.x; Uv = b.y; UE = a.y;
     }
-#pragma unroll 2
+#pragma unroll kUnroll
     for (; m < nrows; ++m) {
         V2 a, b;
         load(m, a, b);

@@ -361,3 +361,27 @@ def test_many_blocks_of_one_row(cuda, T):
             best = min(best, a.elapsed_time(b))
         us.append(best)
     assert us[0] < 3.3 * us[1]
+
+
+@pytest.mark.parametrize("T, blocks", [(np.float64, 5), (np.float32, 8)])
+@pytest.mark.parametrize("arith", ["strict", "fused"])
+def test_other_register_budget_does_not_spill_away(cuda, T, blocks, arith):
+    """The 2D kernels built for more blocks per SM stay near the built-in ones (5 blocks in FP64 took 1.3
+    to 2 times as long where their loop spilled)."""
+    run = hb.BlastRun((8000, 4000), T, arith=arith)
+    dtd = run.phys.dtd(run.dt)
+    best = {}
+    try:
+        for b in (4, blocks, 4, blocks):
+            hb.set_launch_shape(2, T, 0, 0, b)
+            for _ in range(6):
+                e0, e1 = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
+                e0.record()
+                for _ in range(5):
+                    hb.step(run.cur, run.nxt, run.dt_dev, run.phys, dtd, sync=False, arith=arith)
+                e1.record()
+                e1.synchronize()
+                best[b] = min(best.get(b, float("inf")), e0.elapsed_time(e1))
+    finally:
+        hb.set_launch_shape(2, T, 0, 0, 0)
+    assert best[blocks] < (1.2 if arith == "strict" else 1.4) * best[4]
