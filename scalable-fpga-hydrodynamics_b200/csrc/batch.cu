@@ -383,7 +383,7 @@ __device__ __forceinline__ bool publish_item(BatchAcc &acc, ItemPart *parts, int
 
 // The item at hand, its instance's grid and constants, in shared memory: read again where they
 // are needed. Held in registers through the march they cost about 30 of its 128 in 3D FP64, and
-// it spilled: 8 steps of 15.8 M cells took 6.6 ms, so 4.7 ms (5.2 ms with the former march).
+// it spilled: 8 steps of 15.8 M cells took 6.6 ms, so 4.2 ms (5.2 ms with the former march).
 template <class T, class Grid> struct Now {
     int w;   // index of the item
     Item it;

@@ -1,11 +1,14 @@
 // Per-cell arithmetic of the first-order finite-volume update, device side.
 //
-// Every operation is an explicit round-to-nearest intrinsic (__dmul_rn, __dadd_rn,
-// __drcp_rn, __dsqrt_rn, and the float forms), so the compiler can neither contract a
-// multiply and an add into an FMA nor reassociate, whatever -fmad/-use_fast_math say.
-// Each expression keeps the association of the reference source it restates, which
-// makes the results bit-identical to the reference kernel compiled for an IEEE host
-// without contraction (x86-64 SSE2, -ffp-contract=off).
+// Every operation is an explicit round-to-nearest intrinsic (__dmul_rn, __dadd_rn, __fma_rn and
+// the float forms), so the compiler can neither contract a multiply and an add into an FMA
+// nor reassociate, whatever -fmad/-use_fast_math say. Each expression gives the rounded value of
+// the reference source it restates, operation by operation, which makes the results
+// bit-identical to the reference kernel compiled for an IEEE host without contraction (x86-64
+// SSE2, -ffp-contract=off). Where the code is not the reference's operations one by one: the
+// reciprocals and the root of an ordinary cell are correctly rounded by a correction step (Ex
+// below), two products by 1/2 of its conversion are part of an fma (cell2_fast), and the mass
+// flux lacks a "+ 0" (face_flux); each of these says why the values are the same.
 //
 // Faces are computed once per face instead of once per adjacent cell as the reference
 // does (hydro2d/kernel.cxx:186-251 evaluates each face from both sides); the two
@@ -14,8 +17,8 @@
 // sqrt(gamma*p*rho), the upwinded conservative values) are computed once per cell.
 //
 // Every per-cell function takes a template flag kF selecting the arithmetic:
-//  kF = false (strict): the reference's operation order with one rounding per operation,
-//    bit-identical to the reference kernel compiled without contraction;
+//  kF = false (strict): the values of the reference's operation order with one rounding per
+//    operation, bit-identical to the reference kernel compiled without contraction;
 //  kF = true (fused): the same formulas with each product that feeds a sum fused into one
 //    rounding (fma), the reciprocal and square roots from the hardware approximations
 //    refined by one third-order step (Fu below), and the energy of z faces taken from the
@@ -294,7 +297,8 @@ template <class T> struct Cell2 {
 // make_cell2_checked; make_cell2 recomputes such a cell with that, in one branch behind the
 // block. What bounds the marches is issue slots and latency: with the intrinsics' three
 // special-case branches per cell the strict march issued 329 instructions per 2D cell-update
-// at 8000 x 8000 FP64, so 294 (72.5 -> 79.3 GCell/s; FP32 107 -> 118). Recomputing behind the
+// at 8000 x 8000 FP64, so 294 (72.5 -> 79.3 GCell/s; FP32 107 -> 118), and 265 as the march stages
+// its rows now (81.9, FP32 125). Recomputing behind the
 // x face instead keeps more values alive across it: 75.6 GCell/s.
 //
 // Strict: products by 1/2 are exact, so they move into an fma with the sum that follows

@@ -31,11 +31,11 @@
 // instead of eight or ten selects of values in two registers each), which also means that they
 // need not be kept in registers from plane to plane; places in the rings are running offsets;
 // and a wait that gives up is noted in a flag of its thread, not looked up by every thread
-// after every barrier. Per cell-update FP64 strict 484 instructions at 256^3, from 590 (512^3: 39.4 ->
-// 42.7 GCell/s strict, 43.1 -> 45.6 fused; 512 x 512 x 511: 34.0 -> 37.3, 36.7 -> 40.9; FP32
-// 61.4 -> 64.4, 67.6 -> 69.3). Without a second form of the loop for tiles at the walls it also
+// after every barrier. Per cell-update FP64 strict 490 instructions at 256^3, from 590 (512^3: 39.4 ->
+// 42.7 GCell/s strict, 43.1 -> 45.0 fused; 512 x 512 x 511: 34.0 -> 37.7, 36.7 -> 41.1; FP32
+// 61.4 -> 62.9, 67.6 -> 71.2). Without a second form of the loop for tiles at the walls it also
 // stays in the instruction cache where both kinds of tile run side by side: 256^3 FP32 fused
-// 53.4 -> 61.5, 321 x 255 x 259 56.8 -> 63.8, 170^3 FP64 27.5 -> 30.3.
+// 53.4 -> 62.8, 321 x 255 x 259 56.8 -> 65.2, 170^3 FP64 27.5 -> 31.3.
 #pragma once
 
 #include "hydro_rt.cuh"
