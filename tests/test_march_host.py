@@ -6,9 +6,16 @@ import ctypes
 import random
 import subprocess
 
+import pytest
+
 from conftest import ROOT, load_pkg
 
 hb = load_pkg()
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    hb.build()
 
 
 def test_result_of_a_step_by_its_error_bits():
